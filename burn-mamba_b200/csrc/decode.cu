@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(kLinThreads) decode_linear_kernel(const __grid
                 if (j < batch) o[(int64_t)j * n] = __uint_as_float(r[j]) + (PLANES == 2 ? __uint_as_float(r[(ROWS + j) & 15]) : 0.f);
         }
     } else if (tid == 0) {
-        if (status) atomicExch(status, BM_ERR_TIMEOUT);
+        atomicExch(status, BM_ERR_TIMEOUT);
         // copies in flight land in this CTA's shared memory: wait for them (bounded) before it is given back
         for (int i = 0; i < ST; ++i) wait_bounded(&full[i], 0);
     }
@@ -452,6 +452,10 @@ extern "C" int32_t bmx_decode_linear(const void* x, int32_t planes, const void* 
                                      int32_t* status, int32_t first, void* stream) {
     CUtensorMap mw, mx;
     const char* err = nullptr;
+    BM_REQUIRE_PTR(x);
+    BM_REQUIRE_PTR(w);
+    BM_REQUIRE_PTR(part);
+    BM_REQUIRE_PTR(status);
     const uint64_t dw[2] = {(uint64_t)n, (uint64_t)k}, sw[1] = {(uint64_t)n * 2};
     const uint64_t dx[3] = {(uint64_t)k, (uint64_t)batch, (uint64_t)planes}, sx[2] = {(uint64_t)k * 2, (uint64_t)batch * k * 2};
     const uint32_t bw[2] = {64, kLinK}, bx[3] = {kLinK, (uint32_t)(kLinRows / planes), (uint32_t)planes};
@@ -462,11 +466,41 @@ extern "C" int32_t bmx_decode_linear(const void* x, int32_t planes, const void* 
     return planes == 2 ? go(launch_linear<false, 2>) : go(launch_linear<false, 1>);
 }
 
+static int32_t check_rows(const bmx_rows* r) {
+    BM_REQUIRE(r != nullptr, BM_ERR_NULL_POINTER, "rows are NULL");
+    if (r->part) BM_REQUIRE_PTR(r->part);
+    else BM_REQUIRE_PTR(r->dense);
+    return BM_OK;
+}
+static int32_t check_mixer(const bmx_mixer* a) {
+    if (int32_t e = check_rows(&a->proj)) return e;
+    BM_REQUIRE_PTR(a->state);
+    BM_REQUIRE_PTR(a->window);
+    BM_REQUIRE_PTR(a->conv_w);
+    BM_REQUIRE_PTR(a->conv_b);
+    BM_REQUIRE_PTR(a->a);
+    BM_REQUIRE_PTR(a->d);
+    BM_REQUIRE_PTR(a->dt_bias);
+    BM_REQUIRE_PTR(a->gamma);
+    BM_REQUIRE_PTR(a->out);
+    BM_REQUIRE_PTR(a->ss);
+    return BM_OK;
+}
 static unsigned row_threads(int width) { return (unsigned)(cdiv(width, 8 * 32) * 32); }
 
 extern "C" int32_t bmx_decode_norm(const void* residual, const float* residual32, const bmx_rows* add, const bmx_mixer* prev, const void* gamma, float eps,
                                    float* x32, void* x_out, void* out, int32_t planes, int32_t batch, int32_t width, int32_t first, void* stream) {
     using T = __nv_bfloat16;
+    if (add)
+        if (int32_t e = check_rows(add)) return e;
+    if (prev)
+        if (int32_t e = check_mixer(prev)) return e;
+    BM_OPTIONAL_PTR(residual);
+    BM_OPTIONAL_PTR(residual32);
+    BM_OPTIONAL_PTR(x32);
+    BM_OPTIONAL_PTR(x_out);
+    BM_OPTIONAL_PTR(out);
+    if (out) BM_REQUIRE_PTR(gamma);
     const bmx_rows none{};
     const bmx_mixer nomix{};
     return launch_chained("decode_norm", !first, batch, row_threads(width), 0, static_cast<cudaStream_t>(stream), decode_norm_kernel,
@@ -479,20 +513,41 @@ extern "C" int32_t bmx_decode_mixer_sums(int32_t batch, int32_t nheads, int32_t 
     return (int64_t)batch * nheads < kMixPairs ? nheads * (int32_t)cdiv(headdim, kMixRows) : 0;
 }
 extern "C" int32_t bmx_decode_mixer(const bmx_mixer* a, void* stream) {
+    if (int32_t e = check_mixer(a)) return e;
     const int nsplit = (int)cdiv(a->headdim, kMixRows);
     return launch_chained("decode_mixer", true, a->batch * a->nheads * nsplit, 256, 0, static_cast<cudaStream_t>(stream), decode_mixer_kernel, *a, nsplit);
 }
 
 extern "C" int32_t bmx_decode_conv(const bm_conv_step_args* a, const bmx_rows* in, int32_t col, int32_t first, void* stream) {
+    if (int32_t e = check_rows(in)) return e;
+    BM_REQUIRE_PTR(a->window);
+    BM_REQUIRE_PTR(a->weight);
+    BM_OPTIONAL_PTR(a->bias);
+    BM_REQUIRE_PTR(a->out);
+    BM_REQUIRE_PTR(a->out_b);
+    BM_REQUIRE_PTR(a->out_c);
     return launch_chained("decode_conv", !first, dim3((unsigned)cdiv(a->channels, 128), (unsigned)cdiv(a->batch, 2)), 128, 0,
                           static_cast<cudaStream_t>(stream), decode_conv_kernel, *a, *in, col);
 }
 
 extern "C" int32_t bmx_decode_state(const bm_step2_args* a, const bmx_rows* in, int32_t col, void* stream) {
+    if (int32_t e = check_rows(in)) return e;
+    BM_REQUIRE_PTR(a->state);
+    BM_REQUIRE_PTR(a->x);
+    BM_REQUIRE_PTR(a->a);
+    BM_REQUIRE_PTR(a->b);
+    BM_REQUIRE_PTR(a->c);
+    BM_OPTIONAL_PTR(a->d);
+    BM_REQUIRE_PTR(a->dt_bias);
+    BM_REQUIRE_PTR(a->y);
     return launch_step2_rows<__nv_bfloat16>(*a, DtRows{*in, col}, true, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int32_t bmx_decode_gated_norm(const bm_rmsnorm_gated_args* a, const bmx_rows* z, int32_t planes, void* stream) {
+    if (int32_t e = check_rows(z)) return e;
+    BM_REQUIRE_PTR(a->x);
+    BM_REQUIRE_PTR(a->gamma);
+    BM_REQUIRE_PTR(a->out);
     return launch_chained("decode_gated_norm", true, a->rows, row_threads(a->width), 0, static_cast<cudaStream_t>(stream), decode_gated_norm_kernel, *a, *z,
                           planes == 2 ? (int64_t)a->rows * a->width : 0);
 }

@@ -11,6 +11,7 @@
 #include <Python.h>
 
 #include <ATen/ATen.h>
+#include <ATen/TensorSubclassLikeUtils.h>
 #include <ATen/autocast_mode.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/core/GradMode.h>
@@ -81,6 +82,7 @@ std::string shape_str(at::IntArrayRef s) {
 struct Args {
     PyObject* const* a;
     Py_ssize_t n, i = 0;
+    bool exact = true;   // no tensor so far was of a subclass of torch.Tensor
     PyObject* next() {
         if (i >= n) value_error("too few arguments");
         return a[i++];
@@ -112,6 +114,7 @@ struct Args {
             value_error(std::string(name) + " is required");
         }
         if (!THPVariable_Check(o)) value_error(std::string(name) + " must be a torch.Tensor");
+        exact = exact && THPVariable_CheckExact(o);
         return &THPVariable_Unpack(o);
     }
 };
@@ -612,8 +615,14 @@ struct M2Layer {
     int before_gate;
     float dt_min, dt_max;
 };
+// A tensor whose values are what lies at its pointer, for any reader.  Not so: tensors that dispatch elsewhere (subclasses
+// without storage, batched, functional or sparse tensors; everything while a dispatch mode watches), lazy negations, zeros
+// without memory.
+bool plain(const Tensor& t) {
+    return !at::isTensorSubclassLike(t) && t.layout() == at::kStrided && !t.is_neg() && !t._is_zerotensor() && t.has_storage() && t.data_ptr() != nullptr;
+}
 bool dense(const Tensor& t, at::ScalarType dt, at::IntArrayRef shape) {
-    return t.defined() && t.is_cuda() && t.scalar_type() == dt && t.sizes() == shape && t.is_contiguous() &&
+    return t.defined() && t.is_cuda() && plain(t) && t.scalar_type() == dt && t.sizes() == shape && t.is_contiguous() &&
            reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0 && !(c10::GradMode::is_enabled() && t.requires_grad()) && !t._fw_grad(0).defined();
 }
 // Under autocast torch picks the type of every product: the native chains take their operands as they are, so such calls
@@ -626,7 +635,7 @@ bool read_layer(PyObject* tup, int64_t B, int64_t DM, M2Layer& l) {
     if (!PyTuple_Check(tup) || PyTuple_GET_SIZE(tup) != 16) return false;
     for (int i = 0; i < 11; ++i) {
         PyObject* o = PyTuple_GET_ITEM(tup, i);
-        if (THPVariable_Check(o)) *ts[i] = THPVariable_Unpack(o);
+        if (THPVariable_CheckExact(o)) *ts[i] = THPVariable_Unpack(o);   // a subclass may redefine the products: not the chain's
         else if (o != Py_None || i != 10) return false;
     }
     l.H = PyLong_AsLongLong(PyTuple_GET_ITEM(tup, 11)), l.G = PyLong_AsLongLong(PyTuple_GET_ITEM(tup, 12));
@@ -656,7 +665,7 @@ FN(m2_decode) {
     const float eps = (float)A.real();
     if (!PyList_Check(list) || PyList_GET_SIZE(list) == 0 || x.dim() != 2) return none();
     const int64_t B = x.size(0), DM = x.size(1), n = PyList_GET_SIZE(list);
-    if (autocasting() || B < 1 || B > 131070 /* two rows per block of a 65535-wide grid axis */ || !dense(x, at::kBFloat16, {B, DM}) || (residual && !dense(*residual, at::kBFloat16, {B, DM}))) return none();
+    if (!A.exact || autocasting() || B < 1 || B > 131070 /* two rows per block of a 65535-wide grid axis */ || !dense(x, at::kBFloat16, {B, DM}) || (residual && !dense(*residual, at::kBFloat16, {B, DM}))) return none();
     std::vector<M2Layer> ls((size_t)n);
     for (int64_t i = 0; i < n; ++i)
         if (!read_layer(PyList_GET_ITEM(list, i), B, DM, ls[(size_t)i])) return none();
@@ -796,7 +805,7 @@ bool read_m3(PyObject* tup, M3Block& b) {
     if (!PyTuple_Check(tup) || PyTuple_GET_SIZE(tup) != 21) return false;
     for (int i = 0; i < 11; ++i) {
         PyObject* o = PyTuple_GET_ITEM(tup, i);
-        if (THPVariable_Check(o)) *ts[i] = THPVariable_Unpack(o);
+        if (THPVariable_CheckExact(o)) *ts[i] = THPVariable_Unpack(o);
         else if (o != Py_None || i < 8) return false;
     }
     int64_t iv[5];
@@ -843,7 +852,7 @@ FN(m3_forward) {
     const Tensor &u = *A.tensor("u"), *ssm = A.tensor("ssm", true), *k = A.tensor("k", true), *v0 = A.tensor("v", true), *angle = A.tensor("angle", true);
     const int64_t chunk = A.num();
     M3Block b;
-    if (autocasting() || u.dim() != 3 || u.size(1) < 1 || !read_m3(tup, b) || b.g.state_rank % 16) return none();
+    if (!A.exact || autocasting() || u.dim() != 3 || u.size(1) < 1 || !read_m3(tup, b) || b.g.state_rank % 16) return none();
     const int64_t B = u.size(0), S = u.size(1), H = b.g.nheads, P = b.g.headdim, R = b.g.state_rank, M = b.g.mimo_rank;
     if (B < 1 || !dense(u, at::kFloat, {B, S, b.DM}) || (ssm != nullptr && !m3_cache(b, B, ssm, k, v0, angle))) return none();
     if (2 * M * b.g.ngroups * R * 4 > 48 * 1024) return none();
@@ -897,7 +906,7 @@ FN(m3_step) {
     PyObject* tup = A.next();
     const Tensor &u = *A.tensor("u"), *ssm = A.tensor("ssm"), *k = A.tensor("k"), *v = A.tensor("v"), *angle = A.tensor("angle");
     M3Block b;
-    if (autocasting() || u.dim() != 2 || !read_m3(tup, b)) return none();
+    if (!A.exact || autocasting() || u.dim() != 2 || !read_m3(tup, b)) return none();
     const int64_t B = u.size(0);
     b.g.batch = (int32_t)B, b.g.seqlen = 1;
     if (B < 1 || !dense(u, at::kFloat, {B, b.DM}) || !m3_cache(b, B, ssm, k, v, angle) || !L.bmx_m3_step_covers(&b.g)) return none();

@@ -294,18 +294,55 @@ int32_t launch_step(const bmx_m3_block& a, float* state, float* k_state, float* 
 
 unsigned tokens(const bmx_m3_block* a) { return (unsigned)((int64_t)a->batch * a->seqlen); }
 
+// The block's own pointers; a kernel's other operands are checked where it is launched.
+int32_t check_block(const bmx_m3_block* a) {
+    BM_REQUIRE_PTR(a->proj);
+    BM_REQUIRE_PTR(a->dt_bias);
+    BM_REQUIRE_PTR(a->d);
+    BM_REQUIRE_PTR(a->b_norm);
+    BM_REQUIRE_PTR(a->c_norm);
+    BM_REQUIRE_PTR(a->b_bias);
+    BM_REQUIRE_PTR(a->c_bias);
+    BM_OPTIONAL_PTR(a->mimo_x);
+    if (a->mimo_rank > 1) {
+        BM_REQUIRE_PTR(a->mimo_z);
+        BM_REQUIRE_PTR(a->mimo_o);
+    }
+    return BM_OK;
+}
+
 }  // namespace
 
 extern "C" int32_t bmx_m3_coefficients(const bmx_m3_block* a, float* dt, float* da, float* gamma, float* scale, float* v, float* rot, void* stream) {
+    if (int32_t e = check_block(a)) return e;
+    BM_REQUIRE_PTR(dt);
+    BM_REQUIRE_PTR(da);
+    BM_REQUIRE_PTR(gamma);
+    BM_REQUIRE_PTR(scale);
+    BM_REQUIRE_PTR(v);
+    BM_REQUIRE_PTR(rot);
     m3_coefficients_kernel<<<tokens(a), 256, 0, static_cast<cudaStream_t>(stream)>>>(*a, dt, da, gamma, scale, v, rot);
     return check_launch("m3_coefficients");
 }
 extern "C" int32_t bmx_m3_seed(const bmx_m3_block* a, const float* dt, const float* gamma, const float* ssm, const float* k, const float* v, float* h0,
                                void* stream) {
+    if (int32_t e = check_block(a)) return e;
+    BM_REQUIRE_PTR(dt);
+    BM_REQUIRE_PTR(gamma);
+    BM_REQUIRE_PTR(ssm);
+    BM_REQUIRE_PTR(k);
+    BM_REQUIRE_PTR(v);
+    BM_REQUIRE_PTR(h0);
     m3_seed_kernel<<<(unsigned)((int64_t)a->batch * a->nheads), 256, 0, static_cast<cudaStream_t>(stream)>>>(*a, dt, gamma, ssm, k, v, h0);
     return check_launch("m3_seed");
 }
 extern "C" int32_t bmx_m3_tail(const bmx_m3_block* a, const float* y, const float* b_rot, float* out, float* k_last, float* v_last, void* stream) {
+    if (int32_t e = check_block(a)) return e;
+    BM_REQUIRE_PTR(y);
+    BM_REQUIRE_PTR(b_rot);
+    BM_REQUIRE_PTR(out);
+    BM_REQUIRE_PTR(k_last);
+    BM_REQUIRE_PTR(v_last);
     m3_tail_kernel<<<tokens(a), 256, 0, static_cast<cudaStream_t>(stream)>>>(*a, y, b_rot, out, k_last, v_last);
     return check_launch("m3_tail");
 }
@@ -315,6 +352,12 @@ extern "C" int32_t bmx_m3_step_covers(const bmx_m3_block* a) {
     return (m == 1 || m == 2 || m == 4) && a->state_rank % 4 == 0 && a->state_rank <= 128 && a->headdim <= 64 && a->rope_dim <= a->state_rank;
 }
 extern "C" int32_t bmx_m3_step(const bmx_m3_block* a, float* state, float* k_state, float* v_state, float* angle, float* out, void* stream) {
+    if (int32_t e = check_block(a)) return e;
+    BM_REQUIRE_PTR(state);
+    BM_REQUIRE_PTR(k_state);
+    BM_REQUIRE_PTR(v_state);
+    BM_REQUIRE_PTR(angle);
+    BM_REQUIRE_PTR(out);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     switch (a->mimo_rank) {
         case 1: return launch_step<1>(*a, state, k_state, v_state, angle, out, st);
