@@ -621,16 +621,20 @@ struct M2Layer {
 bool plain(const Tensor& t) {
     return !at::isTensorSubclassLike(t) && t.layout() == at::kStrided && !t.is_neg() && !t._is_zerotensor() && t.has_storage() && t.data_ptr() != nullptr;
 }
-bool dense(const Tensor& t, at::ScalarType dt, at::IntArrayRef shape) {
-    return t.defined() && t.is_cuda() && plain(t) && t.scalar_type() == dt && t.sizes() == shape && t.is_contiguous() &&
+// `like`: the activations of the call, on whose device every operand has to be.
+bool dense(const Tensor& t, at::ScalarType dt, at::IntArrayRef shape, const Tensor& like) {
+    return t.defined() && t.is_cuda() && plain(t) && t.device() == like.device() && t.scalar_type() == dt && t.sizes() == shape && t.is_contiguous() &&
            reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0 && !(c10::GradMode::is_enabled() && t.requires_grad()) && !t._fw_grad(0).defined();
 }
+// The chains launch on the current device's stream and read every operand there.
+bool elsewhere(const Tensor& t) { return t.get_device() != c10::cuda::current_device(); }
 // Under autocast torch picks the type of every product: the native chains take their operands as they are, so such calls
 // keep the op-by-op form.
 bool autocasting() { return at::autocast::is_autocast_enabled(at::kCUDA); }
 // Fills `l` from the tuple (w_in, conv_w, conv_b, dt_bias, a, d, gamma, w_out, window, state, norm | None, nheads, ngroups,
 // norm_before_gate, dt_min, dt_max); false when the chain does not cover the layer.
-bool read_layer(PyObject* tup, int64_t B, int64_t DM, M2Layer& l) {
+bool read_layer(PyObject* tup, const Tensor& x, M2Layer& l) {
+    const int64_t B = x.size(0), DM = x.size(1);
     Tensor* ts[] = {&l.w_in, &l.conv_w, &l.conv_b, &l.dt_bias, &l.a, &l.d, &l.gamma, &l.w_out, &l.window, &l.state, &l.norm};
     if (!PyTuple_Check(tup) || PyTuple_GET_SIZE(tup) != 16) return false;
     for (int i = 0; i < 11; ++i) {
@@ -650,9 +654,9 @@ bool read_layer(PyObject* tup, int64_t B, int64_t DM, M2Layer& l) {
     if (l.state.dim() != 4 || l.H < 1 || l.G < 1 || l.H % l.G) return false;
     l.P = l.state.size(2), l.DI = l.H * l.P, l.V = l.DI + 2 * l.G * R, l.N = l.DI + l.V + l.H;
     if (l.DI % 8 || l.N % 8 || DM % 8 || l.DI > 8192 || DM > 8192) return false;
-    return dense(l.w_in, bf, {DM, l.N}) && dense(l.w_out, bf, {l.DI, DM}) && dense(l.gamma, bf, {l.DI}) && dense(l.conv_w, f, {l.V, K}) &&
-           dense(l.conv_b, f, {l.V}) && dense(l.dt_bias, f, {l.H}) && dense(l.a, f, {l.H}) && dense(l.d, f, {l.H}) &&
-           dense(l.window, f, {B, l.V, K}) && dense(l.state, f, {B, l.H, l.P, R}) && (!l.norm.defined() || dense(l.norm, bf, {DM}));
+    return dense(l.w_in, bf, {DM, l.N}, x) && dense(l.w_out, bf, {l.DI, DM}, x) && dense(l.gamma, bf, {l.DI}, x) && dense(l.conv_w, f, {l.V, K}, x) &&
+           dense(l.conv_b, f, {l.V}, x) && dense(l.dt_bias, f, {l.H}, x) && dense(l.a, f, {l.H}, x) && dense(l.d, f, {l.H}, x) &&
+           dense(l.window, f, {B, l.V, K}, x) && dense(l.state, f, {B, l.H, l.P, R}, x) && (!l.norm.defined() || dense(l.norm, bf, {DM}, x));
 }
 
 // layers (list of tuples), x [b, d_model] bf16, residual | None (only without layer norms), eps -> y [b, d_model], or None
@@ -665,14 +669,14 @@ FN(m2_decode) {
     const float eps = (float)A.real();
     if (!PyList_Check(list) || PyList_GET_SIZE(list) == 0 || x.dim() != 2) return none();
     const int64_t B = x.size(0), DM = x.size(1), n = PyList_GET_SIZE(list);
-    if (!A.exact || autocasting() || B < 1 || B > 131070 /* two rows per block of a 65535-wide grid axis */ || !dense(x, at::kBFloat16, {B, DM}) || (residual && !dense(*residual, at::kBFloat16, {B, DM}))) return none();
+    if (!A.exact || autocasting() || B < 1 || B > 131070 /* two rows per block of a 65535-wide grid axis */ || !dense(x, at::kBFloat16, {B, DM}, x) || (residual && !dense(*residual, at::kBFloat16, {B, DM}, x))) return none();
     std::vector<M2Layer> ls((size_t)n);
     for (int64_t i = 0; i < n; ++i)
-        if (!read_layer(PyList_GET_ITEM(list, i), B, DM, ls[(size_t)i])) return none();
+        if (!read_layer(PyList_GET_ITEM(list, i), x, ls[(size_t)i])) return none();
     const bool norms = ls[0].norm.defined();
     for (auto& l : ls)
         if (l.norm.defined() != norms) return none();
-    if (!norms && n != 1) return none();
+    if ((!norms && n != 1) || elsewhere(x)) return none();
     // the chain reads a layer's caches before the kernels of earlier layers have ended: layers that share one run in order
     std::vector<std::pair<uintptr_t, uintptr_t>> spans;
     for (auto& l : ls)
@@ -800,7 +804,7 @@ struct M3Block {
 };
 // Tuple (w_in, dt_bias, d, b_norm, c_norm, b_bias, c_bias, w_out, mimo_x | None, mimo_z | None, mimo_o | None, nheads, state_rank,
 // ngroups, mimo_rank, rope_dim, range, dt_min, dt_max, a_floor, eps); false when the fused kernels do not cover the block.
-bool read_m3(PyObject* tup, M3Block& b) {
+bool read_m3(PyObject* tup, const Tensor& u, M3Block& b) {
     Tensor* ts[] = {&b.w_in, &b.dt_bias, &b.d, &b.b_norm, &b.c_norm, &b.b_bias, &b.c_bias, &b.w_out, &b.mimo_x, &b.mimo_z, &b.mimo_o};
     if (!PyTuple_Check(tup) || PyTuple_GET_SIZE(tup) != 21) return false;
     for (int i = 0; i < 11; ++i) {
@@ -824,9 +828,9 @@ bool read_m3(PyObject* tup, M3Block& b) {
     if (P * H != b.DI || P % 4 || R % 4 || b.N % 4 || b.DI > 1 << 20) return false;
     const auto f = at::kFloat;
     const bool mimo = M > 1;
-    if (!dense(b.w_in, f, {b.DM, b.N}) || !dense(b.w_out, f, {b.DI, b.DM}) || !dense(b.dt_bias, f, {H}) || !dense(b.d, f, {H}) ||
-        !dense(b.b_norm, f, {R}) || !dense(b.c_norm, f, {R}) || !dense(b.b_bias, f, {H, M, R}) || !dense(b.c_bias, f, {H, M, R}) ||
-        (b.mimo_x.defined() && !dense(b.mimo_x, f, {H, M, P})) || (mimo && (!dense(b.mimo_z, f, {H, M, P}) || !dense(b.mimo_o, f, {H, M, P}))))
+    if (!dense(b.w_in, f, {b.DM, b.N}, u) || !dense(b.w_out, f, {b.DI, b.DM}, u) || !dense(b.dt_bias, f, {H}, u) || !dense(b.d, f, {H}, u) ||
+        !dense(b.b_norm, f, {R}, u) || !dense(b.c_norm, f, {R}, u) || !dense(b.b_bias, f, {H, M, R}, u) || !dense(b.c_bias, f, {H, M, R}, u) ||
+        (b.mimo_x.defined() && !dense(b.mimo_x, f, {H, M, P}, u)) || (mimo && (!dense(b.mimo_z, f, {H, M, P}, u) || !dense(b.mimo_o, f, {H, M, P}, u))))
         return false;
     bmx_m3_block& g = b.g;
     memset(&g, 0, sizeof g);
@@ -837,11 +841,12 @@ bool read_m3(PyObject* tup, M3Block& b) {
     g.mimo_z = mimo ? fptr(&b.mimo_z) : nullptr, g.mimo_o = mimo ? fptr(&b.mimo_o) : nullptr;
     return true;
 }
-bool m3_cache(const M3Block& b, int64_t B, const Tensor* ssm, const Tensor* k, const Tensor* v, const Tensor* angle) {
+bool m3_cache(const M3Block& b, const Tensor& u, const Tensor* ssm, const Tensor* k, const Tensor* v, const Tensor* angle) {
     const bmx_m3_block& g = b.g;
     const auto f = at::kFloat;
-    return ssm && k && v && angle && dense(*ssm, f, {B, g.nheads, g.headdim, g.state_rank}) && dense(*k, f, {B, g.mimo_rank, g.nheads, g.state_rank}) &&
-           dense(*v, f, {B, g.nheads, g.headdim}) && dense(*angle, f, {B, g.nheads, b.NA});
+    const int64_t B = u.size(0);
+    return ssm && k && v && angle && dense(*ssm, f, {B, g.nheads, g.headdim, g.state_rank}, u) && dense(*k, f, {B, g.mimo_rank, g.nheads, g.state_rank}, u) &&
+           dense(*v, f, {B, g.nheads, g.headdim}, u) && dense(*angle, f, {B, g.nheads, b.NA}, u);
 }
 
 // block, u [b, s, d_model], ssm | None, k, v, angle, chunk_len -> (out, ssm, k, v, angle), or None when not covered.
@@ -852,10 +857,10 @@ FN(m3_forward) {
     const Tensor &u = *A.tensor("u"), *ssm = A.tensor("ssm", true), *k = A.tensor("k", true), *v0 = A.tensor("v", true), *angle = A.tensor("angle", true);
     const int64_t chunk = A.num();
     M3Block b;
-    if (!A.exact || autocasting() || u.dim() != 3 || u.size(1) < 1 || !read_m3(tup, b) || b.g.state_rank % 16) return none();
+    if (!A.exact || autocasting() || u.dim() != 3 || u.size(1) < 1 || !read_m3(tup, u, b) || b.g.state_rank % 16) return none();
     const int64_t B = u.size(0), S = u.size(1), H = b.g.nheads, P = b.g.headdim, R = b.g.state_rank, M = b.g.mimo_rank;
-    if (B < 1 || !dense(u, at::kFloat, {B, S, b.DM}) || (ssm != nullptr && !m3_cache(b, B, ssm, k, v0, angle))) return none();
-    if (2 * M * b.g.ngroups * R * 4 > 48 * 1024) return none();
+    if (B < 1 || !dense(u, at::kFloat, {B, S, b.DM}, u) || (ssm != nullptr && !m3_cache(b, u, ssm, k, v0, angle))) return none();
+    if (elsewhere(u) || 2 * M * b.g.ngroups * R * 4 > 48 * 1024) return none();
     const auto f = at::kFloat;
     void* st = stream();
     Tensor proj = at::mm(u.view({B * S, b.DM}), b.w_in);
@@ -906,10 +911,10 @@ FN(m3_step) {
     PyObject* tup = A.next();
     const Tensor &u = *A.tensor("u"), *ssm = A.tensor("ssm"), *k = A.tensor("k"), *v = A.tensor("v"), *angle = A.tensor("angle");
     M3Block b;
-    if (!A.exact || autocasting() || u.dim() != 2 || !read_m3(tup, b)) return none();
+    if (!A.exact || autocasting() || u.dim() != 2 || !read_m3(tup, u, b)) return none();
     const int64_t B = u.size(0);
     b.g.batch = (int32_t)B, b.g.seqlen = 1;
-    if (B < 1 || !dense(u, at::kFloat, {B, b.DM}) || !m3_cache(b, B, ssm, k, v, angle) || !L.bmx_m3_step_covers(&b.g)) return none();
+    if (B < 1 || !dense(u, at::kFloat, {B, b.DM}, u) || !m3_cache(b, u, ssm, k, v, angle) || !L.bmx_m3_step_covers(&b.g) || elsewhere(u)) return none();
     Tensor proj = at::mm(u, b.w_in), g = empty({B, b.DI}, at::kFloat, u);
     b.g.proj = fptr(&proj);
     check(L.bmx_m3_step(&b.g, fptr(*ssm), fptr(*k), fptr(*v), fptr(*angle), fptr(g), stream()), "Mamba-3 step");

@@ -92,6 +92,12 @@ def test_chains_leave_python_subclasses_and_lazy_negations_to_the_general_form(b
         assert all(call() is None for call in _calls(bm, kind, make, odd))
 
 
+@pytest.mark.parametrize("kind,odd", OPERANDS)
+def test_chains_leave_operands_on_two_devices_to_the_general_form(bm, kind, odd):
+    """torch refuses such a call in the general form; a chain would read another device's address."""
+    assert all(call() is None for call in _calls(bm, kind, lambda s, d: _plain(s, d, "cuda:1"), odd))
+
+
 def test_entry_points_of_the_chain_kernels_refuse_missing_pointers(bm):
     """A zeroed argument block (all pointers NULL) is refused on the host; nothing is launched."""
     lib, zeros = C.CDLL(bm._ffi.LIB_PATH), C.create_string_buffer(1024)
