@@ -13,6 +13,7 @@
 #include "tc_common.cuh"
 
 #include <algorithm>
+#include <mutex>
 
 using namespace bm;
 
@@ -55,13 +56,14 @@ __device__ __forceinline__ bool wait_bounded(uint64_t* bar, uint32_t parity) {
 
 template <bool DEEP, int PLANES>
 __global__ void __launch_bounds__(kLinThreads) decode_linear_kernel(const __grid_constant__ CUtensorMap mw, const __grid_constant__ CUtensorMap mx,
-                                                                    float* part, int batch, int n, int kblocks, int nslice, int32_t* status) {
+                                                                    float* part, int batch, int n, int kblocks, int nslice, volatile int32_t* status,
+                                                                    int stall) {
     constexpr int ST = lin_stages(DEEP), SB = kLinStageBytes, TCOLS = 32;   // the smallest TMEM allocation
     extern __shared__ __align__(1024) unsigned char raw[];
     unsigned char* base = raw + ((1024u - (tc::smem_u32(raw) & 1023u)) & 1023u);
     __shared__ uint64_t full[ST], empty[ST], done;
     __shared__ uint32_t tmem_slot;
-    __shared__ int gave_up;
+    __shared__ int gave_up, loads;
     const int tid = threadIdx.x, warp = tid >> 5;
     const int col0 = blockIdx.x * kLinCols, s = blockIdx.y;
     const int kb0 = (int)((int64_t)kblocks * s / nslice), nkb = (int)((int64_t)kblocks * (s + 1) / nslice) - kb0;
@@ -90,17 +92,19 @@ __global__ void __launch_bounds__(kLinThreads) decode_linear_kernel(const __grid
             tma_load_2d(st + kLinWBytes / 2, &mw, &full[i % ST], col0 + 64, (kb0 + i) * kLinK);
         };
         auto load_x = [&](int i) { tma_load_3d(base + (i % ST) * SB + kLinWBytes, &mx, &full[i % ST], (kb0 + i) * kLinK, 0, 0); };
-        const int pre = min(ST, nkb);
+        const int pre = stall ? 0 : min(ST, nkb);
         for (int i = 0; i < pre; ++i) load_w(i);   // weights: nothing in the chain writes them
         pdl_wait();                                // x: the predecessor does
         asm volatile("fence.proxy.async;" ::: "memory");
         for (int i = 0; i < pre; ++i) load_x(i);
-        bool ok = true;
+        bool ok = !stall;
+        int issued = pre;
         for (int i = ST; ok && i < nkb; ++i) {
             ok = wait_bounded(&empty[i % ST], (i / ST - 1) & 1);
-            if (ok) load_w(i), load_x(i);
+            if (ok) load_w(i), load_x(i), ++issued;
         }
         if (!ok) gave_up = 1;
+        loads = issued;
     } else if (tid == 32) {
         const uint32_t idesc = tc::umma_idesc_bf16(kLinCols, kLinRows, true, false);
         bool ok = true;
@@ -121,8 +125,7 @@ __global__ void __launch_bounds__(kLinThreads) decode_linear_kernel(const __grid
     }
     __syncwarp();
     pdl_wait();
-    const bool landed = wait_bounded(&done, 0);
-    __syncthreads();
+    const bool landed = __syncthreads_and(wait_bounded(&done, 0));   // one answer for the CTA
     if (landed && !gave_up) {
         tc::tc_fence_after();
         const int c = col0 + tid;
@@ -136,10 +139,18 @@ __global__ void __launch_bounds__(kLinThreads) decode_linear_kernel(const __grid
             for (int j = 0; j < ROWS; ++j)
                 if (j < batch) o[(int64_t)j * n] = __uint_as_float(r[j]) + (PLANES == 2 ? __uint_as_float(r[(ROWS + j) & 15]) : 0.f);
         }
-    } else if (tid == 0) {
-        atomicExch(status, BM_ERR_TIMEOUT);
-        // copies in flight land in this CTA's shared memory: wait for them (bounded) before it is given back
-        for (int i = 0; i < ST; ++i) wait_bounded(&full[i], 0);
+    } else {
+        // What this CTA owes is NaN, so that nothing downstream passes for a result, and the host's status word says why.
+        const int c = col0 + tid;
+        if (c < n)
+            for (int j = 0; j < batch; ++j) part[((int64_t)s * batch + j) * n + c] = __int_as_float(0x7fffffff);
+        if (tid == 0) {
+            *status = BM_ERR_TIMEOUT;
+            __threadfence_system();
+            // copies in flight land in this CTA's shared memory: wait for the last one of every stage (bounded) before it is
+            // given back
+            for (int i = max(0, loads - ST); i < loads; ++i) wait_bounded(&full[i % ST], (i / ST) & 1);
+        }
     }
     tc::tc_fence_before();
     __syncthreads();
@@ -418,7 +429,7 @@ __global__ void __launch_bounds__(128) decode_conv_kernel(bm_conv_step_args a, b
 
 template <bool DEEP, int PLANES>
 int32_t launch_linear(const CUtensorMap& mw, const CUtensorMap& mx, float* part, int batch, int k, int n, int nslice, int32_t* status, bool first,
-                      cudaStream_t st) {
+                      int stall, cudaStream_t st) {
     constexpr size_t smem = (size_t)lin_stages(DEEP) * kLinStageBytes + 1024;
     static uint64_t allowed = 0;   // devices whose shared-memory limit for this kernel is raised
     int dev = 0;
@@ -430,10 +441,38 @@ int32_t launch_linear(const CUtensorMap& mw, const CUtensorMap& mx, float* part,
         if (dev <= 63) __atomic_fetch_or(&allowed, (uint64_t)1 << dev, __ATOMIC_RELAXED);
     }
     return launch_chained("decode_linear", !first, dim3((unsigned)cdiv(n, kLinCols), nslice), kLinThreads, smem, st, decode_linear_kernel<DEEP, PLANES>, mw, mx,
-                          part, batch, n, (int)cdiv(k, kLinK), nslice, status);
+                          part, batch, n, (int)cdiv(k, kLinK), nslice, status, stall);
 }
 
 }  // namespace
+
+// One word per device, in pinned host memory that lives as long as the process: a graph may replay a step at any time, and
+// the host looks at the word without a copy or a synchronisation.
+constexpr int kStatusDevices = 64;
+extern "C" int32_t* bmx_chain_status(int32_t device) {
+    static std::mutex mu;
+    static int32_t* words = nullptr;
+    if (device < 0 || device >= kStatusDevices) {
+        fail(BM_ERR_UNSUPPORTED, "device ordinal %d out of range", device);
+        return nullptr;
+    }
+    std::lock_guard<std::mutex> lock(mu);
+    if (words == nullptr) {
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;   // the first step of a process may be one that is captured
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        void* p = nullptr;
+        const int32_t e = check_cuda(cudaHostAlloc(&p, kStatusDevices * sizeof(int32_t), cudaHostAllocPortable | cudaHostAllocMapped), "cudaHostAlloc(status)");
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        if (e) return nullptr;
+        std::fill_n(static_cast<int32_t*>(p), kStatusDevices, 0);
+        words = static_cast<int32_t*>(p);
+    }
+    return words + device;
+}
+extern "C" int32_t bmx_chain_take_status(int32_t* word) {
+    if (__atomic_exchange_n(word, 0, __ATOMIC_RELAXED) == 0) return BM_OK;
+    return fail(BM_ERR_TIMEOUT, "a bounded wait of a decode step on this device ran out: that step's output and the caches it updated are not valid");
+}
 
 // A CTA takes 128 columns x one slice of K.  Where the columns alone give more than half a wave, two CTAs share an SM and
 // the slices fill those slots; else one CTA per SM with twice the stages (fewer slices for the reader to sum, the same
@@ -449,7 +488,7 @@ extern "C" int32_t bmx_decode_slices(int32_t batch, int32_t k, int32_t n) {
 }
 
 extern "C" int32_t bmx_decode_linear(const void* x, int32_t planes, const void* w, float* part, int32_t batch, int32_t k, int32_t n, int32_t nslice,
-                                     int32_t* status, int32_t first, void* stream) {
+                                     int32_t* status, int32_t first, int32_t stall, void* stream) {
     CUtensorMap mw, mx;
     const char* err = nullptr;
     BM_REQUIRE_PTR(x);
@@ -461,7 +500,7 @@ extern "C" int32_t bmx_decode_linear(const void* x, int32_t planes, const void* 
     const uint32_t bw[2] = {64, kLinK}, bx[3] = {kLinK, (uint32_t)(kLinRows / planes), (uint32_t)planes};
     if (!tc::make_tensor_map_bf16(&mw, w, 2, dw, sw, bw, 128, &err) || !tc::make_tensor_map_bf16(&mx, x, 3, dx, sx, bx, 128, &err))
         return fail(BM_ERR_CUDA, "%s", err);
-    auto go = [&](auto f) { return f(mw, mx, part, batch, k, n, nslice, status, first != 0, static_cast<cudaStream_t>(stream)); };
+    auto go = [&](auto f) { return f(mw, mx, part, batch, k, n, nslice, status, first != 0, stall, static_cast<cudaStream_t>(stream)); };
     if (linear_deep((int)cdiv(n, kLinCols))) return planes == 2 ? go(launch_linear<true, 2>) : go(launch_linear<true, 1>);
     return planes == 2 ? go(launch_linear<false, 2>) : go(launch_linear<false, 1>);
 }

@@ -48,13 +48,18 @@ typedef struct {
     float* ss;             /* [b, nss] partial sums of squares that scale comes from */
 } bmx_mixer;
 
+/* Status of the chains on a device: zero until a bounded wait runs out.  The partial sums of the projection that gave up are
+ * then NaN.  NULL (with the thread's error text set) when there is no such word. */
+int32_t* bmx_chain_status(int32_t device);
+/* Returns what the word holds as a status (BM_OK or an error, reported once) and clears it; does not synchronise. */
+int32_t bmx_chain_take_status(int32_t* word);
 /* Number of K slices the streaming projection cuts a [k, n] weight into for this batch; 0 = the shape is not covered. */
 int32_t bmx_decode_slices(int32_t batch, int32_t k, int32_t n);
 /* `first` below: the kernel opens a chain and is launched plainly.
  * Rows a streaming projection reads are [planes][batch][k]: with two planes, hi and lo bf16 halves of each value.
- * part[s][b][n] = sum over slice s of x[b, k] w[k, n] */
+ * part[s][b][n] = sum over slice s of x[b, k] w[k, n].  `stall` (tests): issue no copies, so that the first wait runs out. */
 int32_t bmx_decode_linear(const void* x, int32_t planes, const void* w, float* part, int32_t batch, int32_t k, int32_t n, int32_t nslice, int32_t* status,
-                          int32_t first, void* stream);
+                          int32_t first, int32_t stall, void* stream);
 /* x' = residual (bf16 or float32) + add (any may be missing); x32 = x_out = x' and out = x' / rms(x') * gamma where the pointers are
  * given.  `prev`: the mixer step that `add` is the out-projection of (its row scale is applied, its B / C windows slide). */
 int32_t bmx_decode_norm(const void* residual, const float* residual32, const bmx_rows* add, const bmx_mixer* prev, const void* gamma, float eps, float* x32,

@@ -42,7 +42,7 @@ namespace {
     X(bm_ssd3_double_bwd) X(bm_step2) X(bm_conv_step) X(bm_conv1d_silu_fwd) X(bm_rmsnorm_gated)                    \
     X(bm_mamba3_bc_prep) X(bm_selscan1_fwd) X(bm_selscan1_fwd_workspace_bytes) X(bm_selscan1_fwd_ws) X(bm_step1)   \
     X(bm_ssd3_fwd_workspace_bytes) X(bm_ssd3_single_fwd) X(bm_ssd3_double_fwd) X(bm_angle_cumsum) X(bm_step3)     \
-    X(bmx_decode_slices) X(bmx_decode_linear) X(bmx_decode_norm) X(bmx_decode_conv) X(bmx_decode_state)            \
+    X(bmx_chain_status) X(bmx_chain_take_status) X(bmx_decode_slices) X(bmx_decode_linear) X(bmx_decode_norm) X(bmx_decode_conv) X(bmx_decode_state)            \
     X(bmx_decode_gated_norm) X(bmx_decode_mixer_sums) X(bmx_decode_mixer)                             \
     X(bmx_m3_coefficients) X(bmx_m3_seed) X(bmx_m3_tail) X(bmx_m3_step_covers) X(bmx_m3_step)
 struct Entry {
@@ -157,9 +157,15 @@ const Tensor& workspace(size_t nbytes, const Tensor& like) {
     Tensor& t = g_ws[{like.get_device(), stream()}];
     if (!t.defined() || (size_t)t.numel() < nbytes) {
         t = empty({(int64_t)std::max<size_t>(nbytes, 256)}, at::kByte, like);
-        t.narrow(0, 0, 256).zero_();   // the status word, which the decode chain only writes when a wait runs out
+        t.narrow(0, 0, 256).zero_();   // the status word, which not every call writes
     }
     return t;
+}
+
+int32_t* chain_status(int device) {
+    int32_t* w = L.bmx_chain_status(device);
+    if (w == nullptr) check(BM_ERR_CUDA, "status word of the decode steps");
+    return w;
 }
 
 PyObject* wrap(Tensor t) { return THPVariable_Wrap(std::move(t)); }
@@ -660,13 +666,15 @@ bool read_layer(PyObject* tup, const Tensor& x, M2Layer& l) {
 }
 
 // layers (list of tuples), x [b, d_model] bf16, residual | None (only without layer norms), eps -> y [b, d_model], or None
-// when the chain does not cover the call (the caller then runs the step kernel by kernel).
+// when the chain does not cover the call (the caller then runs the step kernel by kernel).  A wait that ran out in an earlier
+// step on the device is raised here; with a fifth argument that is true, one of this step (synchronises).
 // With layer norms: x <- x + step(norm(x)) per layer; without: step(x) (+ residual) of the one layer.
 FN(m2_decode) {
     BEGIN
     PyObject* list = A.next();
     const Tensor &x = *A.tensor("x"), *residual = A.tensor("residual", true);
     const float eps = (float)A.real();
+    const bool check_status = A.i < A.n && A.flag();
     if (!PyList_Check(list) || PyList_GET_SIZE(list) == 0 || x.dim() != 2) return none();
     const int64_t B = x.size(0), DM = x.size(1), n = PyList_GET_SIZE(list);
     if (!A.exact || autocasting() || B < 1 || B > 131070 /* two rows per block of a 65535-wide grid axis */ || !dense(x, at::kBFloat16, {B, DM}, x) || (residual && !dense(*residual, at::kBFloat16, {B, DM}, x))) return none();
@@ -716,7 +724,8 @@ FN(m2_decode) {
     auto view = [&](int64_t o, int64_t rows, int64_t cols) {
         return at::from_blob(base + o, {rows, cols}, at::TensorOptions().dtype(at::kBFloat16).device(x.device()));
     };
-    int32_t* status = static_cast<int32_t*>(workspace(256, x).data_ptr());
+    int32_t* status = chain_status(x.get_device());
+    check(L.bmx_chain_take_status(status), "decode step (an earlier one)");
     void* st = stream();
     const void* xres = norms ? x.data_ptr() : residual ? residual->data_ptr() : nullptr;   // the residual stream
     const float* xres32 = nullptr;
@@ -742,7 +751,7 @@ FN(m2_decode) {
             proj.nslice = L.bmx_decode_slices((int32_t)B, (int32_t)DM, (int32_t)l.N);
             proj.slice = B * l.N;
             float* p = reinterpret_cast<float*>(base + o_p1);
-            check(L.bmx_decode_linear(in, norms ? planes : 1, l.w_in.data_ptr(), p, (int32_t)B, (int32_t)DM, (int32_t)l.N, proj.nslice, status, !norms, st), "decode step (in-projection)");
+            check(L.bmx_decode_linear(in, norms ? planes : 1, l.w_in.data_ptr(), p, (int32_t)B, (int32_t)DM, (int32_t)l.N, proj.nslice, status, !norms, 0, st), "decode step (in-projection)");
             proj.part = p;
         } else {
             Tensor po = view(o_p1, B, l.N);
@@ -780,7 +789,7 @@ FN(m2_decode) {
             add = bmx_rows{};
             add.nslice = L.bmx_decode_slices((int32_t)B, (int32_t)l.DI, (int32_t)DM), add.slice = B * DM, add.ld = DM;
             float* p = reinterpret_cast<float*>(base + o_p2);
-            check(L.bmx_decode_linear(base + o_g, planes, l.w_out.data_ptr(), p, (int32_t)B, (int32_t)l.DI, (int32_t)DM, add.nslice, status, 0, st), "decode step (out-projection)");
+            check(L.bmx_decode_linear(base + o_g, planes, l.w_out.data_ptr(), p, (int32_t)B, (int32_t)l.DI, (int32_t)DM, add.nslice, status, 0, 0, st), "decode step (out-projection)");
             add.part = p;
             have_add = true;
         } else if (norms) {
@@ -792,6 +801,10 @@ FN(m2_decode) {
         }
     }
     if (stream_w) check(L.bmx_decode_norm(xres, xres32, &add, fused ? &mix : nullptr, nullptr, eps, nullptr, out.data_ptr(), nullptr, 1, (int32_t)B, (int32_t)DM, 0, st), "decode step (residual)");
+    if (check_status) {
+        c10::cuda::getCurrentCUDAStream().synchronize();
+        check(L.bmx_chain_take_status(status), "decode step");
+    }
     return wrap(out);
     END
 }
@@ -923,10 +936,13 @@ FN(m3_step) {
 }
 
 // ---- module ----------------------------------------------------------------------------------------------------------
-// (no arguments) -> device status of the last SSD call on the current device and stream; 0 when there was none
+// (no arguments) -> device status of the last SSD call on the current device and stream, or of the decode steps on the device;
+// 0 when there was none
 FN(workspace_status) {
     BEGIN
     (void)A;
+    c10::cuda::getCurrentCUDAStream().synchronize();
+    if (const int32_t e = L.bmx_chain_take_status(chain_status((int)c10::cuda::current_device()))) return PyLong_FromLong(e);
     const auto it = g_ws.find({(int)c10::cuda::current_device(), stream()});
     return PyLong_FromLong(it == g_ws.end() ? 0 : L.bm_workspace_status(it->second.data_ptr(), stream()));
     END

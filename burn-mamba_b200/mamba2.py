@@ -152,14 +152,15 @@ class Mamba2:
         return (self.w_in, self._conv_w32, self._conv_b32, self.dt_bias, self._a, self.d, self.norm_gamma, self.w_out, cache.conv_bvk,
                 cache.ssm_bhpr, norm_gamma, self.nheads, self.ngroups, self.norm_before_gate, *self.dt_limit)
 
-    def step(self, input_bm, cache: Optional[Mamba2Cache] = None, residual=None):
+    def step(self, input_bm, cache: Optional[Mamba2Cache] = None, residual=None, check_status=False):
         """Mamba2::step (src/mamba2/mamba2.rs:820-1004) -> (out_bm, cache).  The cache tensors are updated
         in place by the kernels and returned.  `residual` (the layer's skip connection) is added to the output when given.
         bf16 layers with state_rank 128 and 4 conv taps run as one native chain of kernels; anything else kernel by
-        kernel around library GEMMs."""
+        kernel around library GEMMs.  The chain's waits are bounded: a step whose wait ran out gives NaN, and the next step on
+        the device raises BmError, as this one does with `check_status` (which synchronises)."""
         bsz = input_bm.shape[0]
         cache = cache or self.zero_cache(bsz)
-        out = _native.m2_decode([self._chain(cache, None)], input_bm, residual, ops.DIV_EPS[torch.bfloat16])
+        out = _native.m2_decode([self._chain(cache, None)], input_bm, residual, ops.DIV_EPS[torch.bfloat16], check_status)
         if out is not None:
             return out, cache
         proj = input_bm @ self.w_in
@@ -180,16 +181,16 @@ def rms_norm(x, gamma):
     return ops.rmsnorm_gated(x, None, gamma.to(x.dtype))
 
 
-def stack_step(blocks, norm_gammas, caches, x_bm):
+def stack_step(blocks, norm_gammas, caches, x_bm, check_status=False):
     """One decode step through a stack of pre-norm residual layers, the default (no class latents, plain
     residual) path of Layers::step / Layer::step_one (src/modules/layers.rs:427-497,
     src/modules/layer.rs:224-229): x <- x + block.step(norm(x)).  `caches` is one Mamba2Cache per layer,
     updated in place.  Returns the output of the last layer [b, d_model].  Per layer this is six launches
     (norm with the residual sum, in-projection, conv step, state step, gated norm, out-projection), chained so that each
     starts while the one before it runs; none of them depends on the host, so the whole step can be replayed from a
-    CUDA graph.  Stacks the native chain does not cover run layer by layer."""
+    CUDA graph.  Stacks the native chain does not cover run layer by layer.  `check_status` as in `Mamba2.step`."""
     chain = [blk._chain(cache, gamma) for blk, gamma, cache in zip(blocks, norm_gammas, caches)]
-    out = _native.m2_decode(chain, x_bm, None, ops.DIV_EPS[torch.bfloat16])
+    out = _native.m2_decode(chain, x_bm, None, ops.DIV_EPS[torch.bfloat16], check_status)
     if out is not None:
         return out
     for blk, gamma, cache in zip(blocks, norm_gammas, caches):

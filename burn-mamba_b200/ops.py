@@ -17,8 +17,8 @@ PATHS = {"auto": _ffi.BM_PATH_AUTO, "exact": _ffi.BM_PATH_EXACT, "tensor": _ffi.
 
 
 def last_workspace_status():
-    """Device status word left by the most recent SSD launch on the current device and stream (synchronises);
-    0 when no launch has used a workspace yet."""
+    """Device status word left by the most recent SSD launch on the current device and stream, or BM_ERR_TIMEOUT when a wait of
+    a decode step on the device ran out and that has not been raised yet (synchronises); 0 when there is nothing to report."""
     return _native.workspace_status()
 
 

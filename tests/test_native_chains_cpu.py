@@ -107,7 +107,7 @@ def test_entry_points_of_the_chain_kernels_refuse_missing_pointers(bm):
     assert lib.bmx_m3_seed(zeros, *[buf] * 6, p()) == null
     assert lib.bmx_m3_tail(zeros, *[buf] * 5, p()) == null
     assert lib.bmx_m3_step(zeros, *[buf] * 5, p()) == null
-    assert lib.bmx_decode_linear(buf, 1, p(), buf, 1, 128, 128, 1, buf, 1, p()) == null
+    assert lib.bmx_decode_linear(buf, 1, p(), buf, 1, 128, 128, 1, buf, 1, 0, p()) == null
     assert lib.bmx_decode_norm(buf, p(), p(), p(), p(), C.c_float(1e-5), p(), p(), buf, 1, 1, 128, 1, p()) == null
     assert lib.bmx_decode_mixer(zeros, p()) == null
     assert lib.bmx_decode_state(zeros, zeros, 0, p()) == null
