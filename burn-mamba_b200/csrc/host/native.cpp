@@ -7,7 +7,8 @@
 //
 // Every function takes its arguments by position (the Python wrappers own names, defaults and documentation) and
 // raises what the wrappers' documentation promises: ValueError for a tensor that does not fit, BmError for a status
-// the library returns.
+// the library returns.  Everything that may block (launches into a full queue, allocations, synchronisation) runs without the
+// GIL, like torch's own operators; what is shared between calls is guarded by its own locks.
 #include <Python.h>
 
 #include <ATen/ATen.h>
@@ -24,6 +25,8 @@
 #include <algorithm>
 #include <cstring>
 #include <map>
+#include <mutex>
+#include <optional>
 #include <string>
 #include <utility>
 #include <vector>
@@ -52,22 +55,47 @@ struct Entry {
 } L;
 PyObject* g_bm_error = nullptr;   // _ffi.BmError
 
-[[noreturn]] void value_error(const std::string& msg) {
-    PyErr_SetString(PyExc_ValueError, msg.c_str());
+// Failures travel as C++ exceptions, which need no GIL, and become Python's where a function ends (END below).
+struct BadValue {
+    std::string msg;
+};
+struct BadStatus {
+    int32_t code;
+    std::string where;
+};
+[[noreturn]] void value_error(const std::string& msg) { throw BadValue{msg}; }
+void check(int32_t code, const char* where) {
+    if (code != BM_OK) throw BadStatus{code, where};
+}
+[[noreturn]] void rethrow_python() {
     python_error e;
     e.persist();
     throw e;
 }
-void check(int32_t code, const char* where) {
-    if (code == BM_OK) return;
-    PyObject* exc = PyObject_CallFunction(g_bm_error, "is", (int)code, where);   // reads the thread's error string
+[[noreturn]] void raise(const BadValue& f) {
+    PyErr_SetString(PyExc_ValueError, f.msg.c_str());
+    rethrow_python();
+}
+[[noreturn]] void raise(const BadStatus& f) {
+    PyObject* exc = PyObject_CallFunction(g_bm_error, "is", (int)f.code, f.where.c_str());   // reads the thread's error string
     if (exc != nullptr) {
         PyErr_SetObject(g_bm_error, exc);
         Py_DECREF(exc);
     }
-    python_error e;
-    e.persist();
-    throw e;
+    rethrow_python();
+}
+
+// A scope without the GIL.  Tensors that Python can reach are only read in one.
+struct NoGil {
+    PyThreadState* state = PyEval_SaveThread();
+    NoGil() = default;
+    NoGil(const NoGil&) = delete;
+    ~NoGil() { PyEval_RestoreThread(state); }
+};
+template <typename F>
+void launch(const char* where, F f) {
+    NoGil scope;
+    check(f(), where);
 }
 
 // ---- argument access ------------------------------------------------------------------------------------------
@@ -89,20 +117,12 @@ struct Args {
     }
     int64_t num() {
         const int64_t v = PyLong_AsLongLong(next());
-        if (v == -1 && PyErr_Occurred()) {
-            python_error e;
-            e.persist();
-            throw e;
-        }
+        if (v == -1 && PyErr_Occurred()) rethrow_python();
         return v;
     }
     double real() {
         const double v = PyFloat_AsDouble(next());
-        if (v == -1.0 && PyErr_Occurred()) {
-            python_error e;
-            e.persist();
-            throw e;
-        }
+        if (v == -1.0 && PyErr_Occurred()) rethrow_python();
         return v;
     }
     bool flag() { return PyObject_IsTrue(next()) == 1; }
@@ -151,15 +171,38 @@ Tensor empty(at::IntArrayRef size, at::ScalarType dtype, const Tensor& like) {
 void* stream() { return static_cast<void*>(c10::cuda::getCurrentCUDAStream().stream()); }
 
 // Grow-only scratch per (device, stream): the C ABI never allocates.  A buffer belongs to its stream, so launches that
-// share it are ordered; there are at most as many entries as streams the program runs the library on.  Guarded by the GIL.
-std::map<std::pair<int, void*>, Tensor> g_ws;
-const Tensor& workspace(size_t nbytes, const Tensor& like) {
-    Tensor& t = g_ws[{like.get_device(), stream()}];
-    if (!t.defined() || (size_t)t.numel() < nbytes) {
-        t = empty({(int64_t)std::max<size_t>(nbytes, 256)}, at::kByte, like);
-        t.narrow(0, 0, 256).zero_();   // the status word, which not every call writes
+// share it are ordered; there are at most as many entries as streams the program runs the library on.  `m` is held while a
+// call's launches go out: the kernels of two threads' calls on one stream would otherwise use the buffer in turns.
+struct Workspace {
+    std::mutex m;
+    Tensor t;
+};
+std::mutex g_ws_mutex;
+std::map<std::pair<int, void*>, Workspace> g_ws;   // entries are never removed
+Workspace* find_workspace(int device, bool create) {
+    const std::pair<int, void*> key{device, stream()};
+    std::lock_guard<std::mutex> lock(g_ws_mutex);
+    if (create) return &g_ws[key];
+    const auto it = g_ws.find(key);
+    return it == g_ws.end() ? nullptr : &it->second;
+}
+// f(workspace, bytes): one call of the library with a workspace of at least `nbytes`; with `status_where`, its device status
+// as well (synchronises).
+template <typename F>
+void with_workspace(size_t nbytes, const Tensor& like, const char* where, const char* status_where, F f) {   // without the GIL
+    Workspace& w = *find_workspace(like.get_device(), true);
+    std::lock_guard<std::mutex> lock(w.m);
+    if (!w.t.defined() || (size_t)w.t.numel() < nbytes) {
+        w.t = empty({(int64_t)std::max<size_t>(nbytes, 256)}, at::kByte, like);
+        w.t.narrow(0, 0, 256).zero_();   // the status word, which not every call writes
     }
-    return t;
+    check(f(w.t.data_ptr(), (size_t)w.t.numel()), where);
+    if (status_where != nullptr) check(L.bm_workspace_status(w.t.data_ptr(), stream()), status_where);
+}
+template <typename F>
+void launch_ws(size_t nbytes, const Tensor& like, const char* where, const char* status_where, F f) {
+    NoGil scope;
+    with_workspace(nbytes, like, where, status_where, f);
 }
 
 int32_t* chain_status(int device) {
@@ -190,6 +233,7 @@ const void* rows(const Tensor& t, const char* name, int64_t* stride, Tensor* kee
     const Tensor* src = &t;
     *stride = d >= 2 ? t.stride(-2) : t.size(-1);
     if ((*stride * (int64_t)t.element_size()) % 16 || reinterpret_cast<uintptr_t>(t.data_ptr()) % 16) {
+        NoGil scope;
         *keep = t.contiguous();
         if (keep->data_ptr() == t.data_ptr()) *keep = t.clone();   // contiguous, yet its base is not aligned
         src = keep;
@@ -202,8 +246,19 @@ const void* rows(const Tensor& t, const char* name, int64_t* stride, Tensor* kee
 }
 
 #define FN(name) PyObject* name(PyObject*, PyObject* const* argv, Py_ssize_t nargs)
-#define BEGIN HANDLE_TH_ERRORS Args A{argv, nargs};
-#define END END_HANDLE_TH_ERRORS
+#define BEGIN        \
+    HANDLE_TH_ERRORS \
+    try {            \
+        Args A{argv, nargs};
+#define END                       \
+    }                             \
+    catch (const BadValue& f) {   \
+        raise(f);                 \
+    }                             \
+    catch (const BadStatus& f) {  \
+        raise(f);                 \
+    }                             \
+    END_HANDLE_TH_ERRORS
 
 // ---- Mamba-2 SSD -----------------------------------------------------------------------------------------------
 // x, dt, a, b, c, d, h0, dt_bias, z, chunk_len, path, dt_min, dt_max, return_states, check_status, reserved, noalloc
@@ -235,11 +290,10 @@ FN(ssd2_fwd) {
     g.dt_bias = fptr(dt_bias), g.z = vptr(z), g.y = y.data_ptr(), g.h_final = fptr(hf);
     g.chunk_states = want_states ? fptr(states) : nullptr;
     if (noalloc) {
-        check(L.bm_ssd2_fwd_noalloc(&g, stream()), "bm_ssd2_fwd_noalloc");
+        launch("bm_ssd2_fwd_noalloc", [&] { return L.bm_ssd2_fwd_noalloc(&g, stream()); });
     } else {
-        const Tensor& ws = workspace(L.bm_ssd2_fwd_workspace_bytes(&g), x);
-        check(L.bm_ssd2_fwd(&g, ws.data_ptr(), (size_t)ws.numel(), stream()), "bm_ssd2_fwd");
-        if (check_status) check(L.bm_workspace_status(ws.data_ptr(), stream()), "bm_ssd2_fwd (device status)");
+        launch_ws(L.bm_ssd2_fwd_workspace_bytes(&g), x, "bm_ssd2_fwd", check_status ? "bm_ssd2_fwd (device status)" : nullptr,
+                  [&](void* ws, size_t n) { return L.bm_ssd2_fwd(&g, ws, n, stream()); });
     }
     if (want_states) return tuple({wrap(y), wrap(hf), wrap(states)});
     return tuple({wrap(y), wrap(hf)});
@@ -271,9 +325,8 @@ FN(ssd2_bwd) {
     g.x = x.data_ptr(), g.dt = fptr(dt), g.a = fptr(a), g.b = b.data_ptr(), g.c = vptr(c), g.d = fptr(d), g.h0 = fptr(h0);
     g.dy = vptr(dy), g.dh_final = fptr(dhf), g.dx = fptr(dx), g.ddt = fptr(ddt), g.da = fptr(da), g.db = fptr(db), g.dc = fptr(dc);
     g.dd = d == nullptr ? nullptr : fptr(dd), g.dh0 = fptr(dh0);
-    const Tensor& ws = workspace(L.bm_ssd2_bwd_workspace_bytes(&g), x);
-    check(L.bm_ssd2_bwd(&g, ws.data_ptr(), (size_t)ws.numel(), stream()), "bm_ssd2_bwd");
-    if (check_status) check(L.bm_workspace_status(ws.data_ptr(), stream()), "bm_workspace_status");
+    launch_ws(L.bm_ssd2_bwd_workspace_bytes(&g), x, "bm_ssd2_bwd", check_status ? "bm_workspace_status" : nullptr,
+              [&](void* ws, size_t n) { return L.bm_ssd2_bwd(&g, ws, n, stream()); });
     PyObject* out = PyDict_New();
     put(out, "dx", wrap(dx)), put(out, "ddt", wrap(ddt)), put(out, "da", wrap(da)), put(out, "db", wrap(db)), put(out, "dc", wrap(dc));
     put(out, "dd", d == nullptr ? none() : wrap(dd)), put(out, "dh0", wrap(dh0));
@@ -300,7 +353,7 @@ FN(step2) {
     g.batch = (int32_t)B, g.nheads = (int32_t)H, g.headdim = (int32_t)P, g.state_rank = (int32_t)R, g.ngroups = (int32_t)G;
     g.state = fptr(st), g.x = x.data_ptr(), g.dt = fptr(dt), g.a = fptr(a), g.b = b.data_ptr(), g.c = vptr(c), g.d = fptr(d);
     g.dt_bias = fptr(dt_bias), g.z = vptr(z), g.y = y.data_ptr();
-    check(L.bm_step2(&g, stream()), "bm_step2");
+    launch("bm_step2", [&] { return L.bm_step2(&g, stream()); });
     return wrap(y);
     END
 }
@@ -342,7 +395,7 @@ FN(conv_step) {
     g.batch = (int32_t)B, g.channels = (int32_t)V, g.kernel = (int32_t)K, g.window = fptr(win), g.xin = xin.data_ptr();
     g.weight = fptr(w), g.bias = fptr(bias), g.out = o.data_ptr(), g.xin_stride = (int32_t)xin.stride(0);
     g.split_x = (int32_t)s.sx, g.split_bc = (int32_t)s.sbc;
-    check(L.bm_conv_step(&g, stream()), "bm_conv_step");
+    launch("bm_conv_step", [&] { return L.bm_conv_step(&g, stream()); });
     return s.on ? tuple({wrap(o), wrap(ob), wrap(oc)}) : wrap(o);
     END
 }
@@ -376,7 +429,7 @@ FN(conv1d_silu_fwd) {
     g.batch = (int32_t)B, g.seqlen = (int32_t)S, g.channels = (int32_t)V, g.kernel = (int32_t)K, g.xin_stride = (int32_t)stride;
     g.split_x = (int32_t)s.sx, g.split_bc = (int32_t)s.sbc, g.weight = fptr(w), g.bias = fptr(bias), g.window = fptr(win);
     g.new_window = want_window ? fptr(nw) : nullptr, g.out_x = o.data_ptr();
-    check(L.bm_conv1d_silu_fwd(&g, stream()), "bm_conv1d_silu_fwd");
+    launch("bm_conv1d_silu_fwd", [&] { return L.bm_conv1d_silu_fwd(&g, stream()); });
     PyObject* outs = s.on ? tuple({wrap(o), wrap(ob), wrap(oc)}) : wrap(o);
     return tuple({outs, want_window ? wrap(nw) : none()});
     END
@@ -401,7 +454,7 @@ FN(rmsnorm_gated) {
     Tensor out = empty(x.sizes(), act, x);
     g.rows = (int32_t)(out.numel() / d), g.width = (int32_t)d, g.x_stride = (int32_t)xs, g.z_stride = (int32_t)zs;
     g.gamma = vptr(gamma), g.out = out.data_ptr();
-    check(L.bm_rmsnorm_gated(&g, stream()), "bm_rmsnorm_gated");
+    launch("bm_rmsnorm_gated", [&] { return L.bm_rmsnorm_gated(&g, stream()); });
     return wrap(out);
     END
 }
@@ -428,10 +481,10 @@ FN(selscan1_fwd) {
     g.u = u.data_ptr(), g.delta = vptr(delta), g.a = fptr(&a), g.b = vptr(b), g.c = vptr(c), g.d = fptr(d), g.delta_bias = fptr(db);
     g.z = vptr(z), g.h0 = fptr(h0), g.y = y.data_ptr(), g.h_final = fptr(hf);
     if (serial) {
-        check(L.bm_selscan1_fwd(&g, stream()), "bm_selscan1_fwd");
+        launch("bm_selscan1_fwd", [&] { return L.bm_selscan1_fwd(&g, stream()); });
     } else {
-        const Tensor& ws = workspace(L.bm_selscan1_fwd_workspace_bytes(&g), u);
-        check(L.bm_selscan1_fwd_ws(&g, ws.data_ptr(), (size_t)ws.numel(), stream()), "bm_selscan1_fwd_ws");
+        launch_ws(L.bm_selscan1_fwd_workspace_bytes(&g), u, "bm_selscan1_fwd_ws", nullptr,
+                  [&](void* ws, size_t n) { return L.bm_selscan1_fwd_ws(&g, ws, n, stream()); });
     }
     return tuple({wrap(y), wrap(hf)});
     END
@@ -456,7 +509,7 @@ FN(step1) {
     g.batch = (int32_t)B, g.d_inner = (int32_t)I, g.state_rank = (int32_t)R;
     g.state = fptr(st), g.u = u.data_ptr(), g.delta = vptr(delta), g.a = fptr(a), g.b = vptr(b), g.c = vptr(c), g.d = fptr(d);
     g.delta_bias = fptr(db), g.z = vptr(z), g.y = y.data_ptr();
-    check(L.bm_step1(&g, stream()), "bm_step1");
+    launch("bm_step1", [&] { return L.bm_step1(&g, stream()); });
     return wrap(y);
     END
 }
@@ -492,7 +545,7 @@ FN(mamba3_bc_prep) {
     g.state_rank = (int32_t)R, g.raw_stride = (int32_t)bs, g.rope_dim = (int32_t)rope, g.pairwise = (int32_t)pairwise, g.eps = (float)eps;
     g.b_gamma = fptr(bg), g.c_gamma = fptr(cg), g.b_bias = fptr(&bb), g.c_bias = fptr(cb), g.angles = fptr(ang);
     g.b_out = ob.data_ptr(), g.c_out = oc.data_ptr();
-    check(L.bm_mamba3_bc_prep(&g, stream()), "bm_mamba3_bc_prep");
+    launch("bm_mamba3_bc_prep", [&] { return L.bm_mamba3_bc_prep(&g, stream()); });
     return tuple({wrap(ob), wrap(oc)});
     END
 }
@@ -520,10 +573,9 @@ FN(ssd3_fwd) {
     g.mimo_rank = (int32_t)M;
     g.v = v.data_ptr(), g.da = fptr(da), g.b = b.data_ptr(), g.c = vptr(c), g.gamma = fptr(gamma), g.scale = fptr(scale);
     g.h0 = fptr(h0), g.angles = fptr(ang), g.y = y.data_ptr(), g.h_final = fptr(hf);
-    const char* name = single ? "bm_ssd3_single_fwd" : "bm_ssd3_double_fwd";
-    const Tensor& ws = workspace(L.bm_ssd3_fwd_workspace_bytes(&g), v);
-    check((single ? L.bm_ssd3_single_fwd : L.bm_ssd3_double_fwd)(&g, ws.data_ptr(), (size_t)ws.numel(), stream()), name);
-    if (check_status) check(L.bm_workspace_status(ws.data_ptr(), stream()), (std::string(name) + " (device status)").c_str());
+    const std::string name = single ? "bm_ssd3_single_fwd" : "bm_ssd3_double_fwd", status_name = name + " (device status)";
+    launch_ws(L.bm_ssd3_fwd_workspace_bytes(&g), v, name.c_str(), check_status ? status_name.c_str() : nullptr,
+              [&](void* ws, size_t n) { return (single ? L.bm_ssd3_single_fwd : L.bm_ssd3_double_fwd)(&g, ws, n, stream()); });
     return tuple({wrap(y), wrap(hf)});
     END
 }
@@ -556,9 +608,8 @@ FN(ssd3_bwd) {
     g.mimo_rank = (int32_t)M;
     g.v = v.data_ptr(), g.da = fptr(da), g.b = b.data_ptr(), g.c = vptr(c), g.h0 = fptr(h0), g.dy = vptr(dy), g.dh_final = fptr(dhf);
     g.dv = fptr(dv), g.dda = fptr(dda), g.db = fptr(db), g.dc = fptr(dc), g.dh0 = fptr(dh0);
-    const Tensor& ws = workspace(L.bm_ssd3_bwd_workspace_bytes(&g), v);
-    check((single ? L.bm_ssd3_single_bwd : L.bm_ssd3_double_bwd)(&g, ws.data_ptr(), (size_t)ws.numel(), stream()), "bm_ssd3_bwd");
-    if (check_status) check(L.bm_workspace_status(ws.data_ptr(), stream()), "bm_workspace_status");
+    launch_ws(L.bm_ssd3_bwd_workspace_bytes(&g), v, "bm_ssd3_bwd", check_status ? "bm_workspace_status" : nullptr,
+              [&](void* ws, size_t n) { return (single ? L.bm_ssd3_single_bwd : L.bm_ssd3_double_bwd)(&g, ws, n, stream()); });
     PyObject* out = PyDict_New();
     put(out, "dv", wrap(dv)), put(out, "dda", wrap(dda)), put(out, "db", wrap(db)), put(out, "dc", wrap(dc)), put(out, "dh0", wrap(dh0));
     if (single) put(out, "dgamma", wrap(dgamma)), put(out, "dscale", wrap(dscale));
@@ -579,7 +630,7 @@ FN(angle_cumsum) {
     Tensor theta = empty({B, S, H, NA}, at::kFloat, rot), last = empty({B, H, NA}, at::kFloat, rot);
     g.batch = (int32_t)B, g.seqlen = (int32_t)S, g.nheads = (int32_t)H, g.nangles = (int32_t)NA;
     g.rot = fptr(&rot), g.dt = fptr(&dt), g.prev = fptr(prev), g.theta = fptr(theta), g.last = fptr(last);
-    check(L.bm_angle_cumsum(&g, stream()), "bm_angle_cumsum");
+    launch("bm_angle_cumsum", [&] { return L.bm_angle_cumsum(&g, stream()); });
     return tuple({wrap(theta), wrap(last)});
     END
 }
@@ -609,7 +660,7 @@ FN(step3) {
     g.rope_dim = (int32_t)rope;
     g.state = fptr(st), g.k_state = fptr(ks), g.v_state = fptr(vs), g.angle = fptr(ang), g.x = fptr(x), g.b = fptr(&b), g.c = fptr(c);
     g.rot = fptr(rot), g.dt = fptr(dt), g.alpha = fptr(al), g.beta = fptr(be), g.gamma = fptr(ga), g.mimo_x = fptr(mx), g.y = fptr(y);
-    check(L.bm_step3(&g, stream()), "bm_step3");
+    launch("bm_step3", [&] { return L.bm_step3(&g, stream()); });
     return wrap(y);
     END
 }
@@ -724,6 +775,8 @@ FN(m2_decode) {
     auto view = [&](int64_t o, int64_t rows, int64_t cols) {
         return at::from_blob(base + o, {rows, cols}, at::TensorOptions().dtype(at::kBFloat16).device(x.device()));
     };
+    std::optional<NoGil> scope;   // until the result is wrapped
+    scope.emplace();
     int32_t* status = chain_status(x.get_device());
     check(L.bmx_chain_take_status(status), "decode step (an earlier one)");
     void* st = stream();
@@ -805,6 +858,7 @@ FN(m2_decode) {
         c10::cuda::getCurrentCUDAStream().synchronize();
         check(L.bmx_chain_take_status(status), "decode step");
     }
+    scope.reset();
     return wrap(out);
     END
 }
@@ -875,6 +929,8 @@ FN(m3_forward) {
     if (B < 1 || !dense(u, at::kFloat, {B, S, b.DM}, u) || (ssm != nullptr && !m3_cache(b, u, ssm, k, v0, angle))) return none();
     if (elsewhere(u) || 2 * M * b.g.ngroups * R * 4 > 48 * 1024) return none();
     const auto f = at::kFloat;
+    std::optional<NoGil> scope;   // until the results are wrapped
+    scope.emplace();
     void* st = stream();
     Tensor proj = at::mm(u.view({B * S, b.DM}), b.w_in);
     b.g.batch = (int32_t)B, b.g.seqlen = (int32_t)S, b.g.proj = fptr(&proj);
@@ -908,11 +964,11 @@ FN(m3_forward) {
     fa.batch = (int32_t)B, fa.seqlen = (int32_t)S, fa.nheads = (int32_t)H, fa.headdim = (int32_t)P, fa.state_rank = (int32_t)R, fa.mimo_rank = (int32_t)M;
     fa.chunk_len = (int32_t)chunk, fa.dtype = BM_DTYPE_F32, fa.v = fptr(v), fa.da = da, fa.b = fptr(bm), fa.c = fptr(cm), fa.gamma = gamma, fa.scale = scale;
     fa.h0 = ssm ? fptr(&h0) : nullptr, fa.y = fptr(y), fa.h_final = fptr(hf);
-    const Tensor& ws = workspace(L.bm_ssd3_fwd_workspace_bytes(&fa), u);
-    check(L.bm_ssd3_single_fwd(&fa, ws.data_ptr(), (size_t)ws.numel(), st), "bm_ssd3_single_fwd");
+    with_workspace(L.bm_ssd3_fwd_workspace_bytes(&fa), u, "bm_ssd3_single_fwd", nullptr, [&](void* ws, size_t n) { return L.bm_ssd3_single_fwd(&fa, ws, n, st); });
     Tensor g = empty({B * S, b.DI}, f, u), kl = empty({B, M, H, R}, f, u), vl = empty({B, H, P}, f, u);
     check(L.bmx_m3_tail(&b.g, fptr(&y), fptr(&bm), fptr(g), fptr(kl), fptr(vl), st), "Mamba-3 block (gate)");
     Tensor out = at::mm(g, b.w_out).view({B, S, b.DM});
+    scope.reset();
     return tuple({wrap(out), wrap(hf), wrap(kl), wrap(vl), wrap(last)});
     END
 }
@@ -928,10 +984,15 @@ FN(m3_step) {
     const int64_t B = u.size(0);
     b.g.batch = (int32_t)B, b.g.seqlen = 1;
     if (B < 1 || !dense(u, at::kFloat, {B, b.DM}, u) || !m3_cache(b, u, ssm, k, v, angle) || !L.bmx_m3_step_covers(&b.g) || elsewhere(u)) return none();
-    Tensor proj = at::mm(u, b.w_in), g = empty({B, b.DI}, at::kFloat, u);
-    b.g.proj = fptr(&proj);
-    check(L.bmx_m3_step(&b.g, fptr(*ssm), fptr(*k), fptr(*v), fptr(*angle), fptr(g), stream()), "Mamba-3 step");
-    return wrap(at::mm(g, b.w_out));
+    Tensor out;
+    {
+        NoGil scope;
+        Tensor proj = at::mm(u, b.w_in), g = empty({B, b.DI}, at::kFloat, u);
+        b.g.proj = fptr(&proj);
+        check(L.bmx_m3_step(&b.g, fptr(*ssm), fptr(*k), fptr(*v), fptr(*angle), fptr(g), stream()), "Mamba-3 step");
+        out = at::mm(g, b.w_out);
+    }
+    return wrap(out);
     END
 }
 
@@ -941,10 +1002,18 @@ FN(m3_step) {
 FN(workspace_status) {
     BEGIN
     (void)A;
-    c10::cuda::getCurrentCUDAStream().synchronize();
-    if (const int32_t e = L.bmx_chain_take_status(chain_status((int)c10::cuda::current_device()))) return PyLong_FromLong(e);
-    const auto it = g_ws.find({(int)c10::cuda::current_device(), stream()});
-    return PyLong_FromLong(it == g_ws.end() ? 0 : L.bm_workspace_status(it->second.data_ptr(), stream()));
+    int32_t status = BM_OK;
+    {
+        NoGil scope;
+        const int device = (int)c10::cuda::current_device();
+        c10::cuda::getCurrentCUDAStream().synchronize();
+        status = L.bmx_chain_take_status(chain_status(device));
+        if (Workspace* w = status == BM_OK ? find_workspace(device, false) : nullptr) {
+            std::lock_guard<std::mutex> lock(w->m);
+            if (w->t.defined()) status = L.bm_workspace_status(w->t.data_ptr(), stream());
+        }
+    }
+    return PyLong_FromLong(status);
     END
 }
 
