@@ -50,11 +50,15 @@ struct Columns {   // column offsets of the projection row
         na = max(a.rope_dim / 2, 1);
     }
 };
+// Clamps that keep NaN, as the reference's do; fminf and fmaxf would drop it.
+__device__ __forceinline__ float at_least(float x, float lo) { return x < lo ? lo : x; }
+__device__ __forceinline__ float at_most(float x, float hi) { return x > hi ? hi : x; }
+
 struct Trapezoid {   // src/mamba3/helpers.rs:42-73
     float dt, da, lam;
     __device__ __forceinline__ Trapezoid(const bmx_m3_block& a, float dd_dt, float dd_a, float lam_raw, float bias) {
-        dt = fminf(fmaxf(softplus_f32(dd_dt + bias), a.dt_min), a.dt_max);
-        da = -dt * fmaxf(softplus_f32(dd_a), a.a_floor);
+        dt = at_most(at_least(softplus_f32(dd_dt + bias), a.dt_min), a.dt_max);
+        da = -dt * at_least(softplus_f32(dd_a), a.a_floor);
         lam = 1.f / (1.f + expf(-lam_raw));
     }
 };

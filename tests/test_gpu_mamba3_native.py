@@ -59,3 +59,26 @@ def test_native_forward_matches_the_unfused_block(bm, monkeypatch, s, m, r, p, r
     assert _close(got, want)
     for k in wc:
         assert gc[k].shape == wc[k].shape and _close(gc[k], wc[k])
+
+
+@pytest.mark.parametrize("value", [float("nan"), float("inf"), float("-inf")])
+@pytest.mark.parametrize("where", ["dt_bias", "dd_dt", "dd_A", "lambda", "rot"])
+def test_infinities_and_nan_reach_the_output_as_in_the_unfused_block(bm, monkeypatch, where, value):
+    """One head's scalar (or one angle) is infinite or NaN: clamps keep NaN, and every value that stays finite is the same."""
+    blk, n = _block(bm, 2, 64, 32, 16, 32, seed=4)
+    at = {"dd_dt": sum(blk.splits[:4]), "dd_A": sum(blk.splits[:5]), "lambda": sum(blk.splits[:6]), "rot": sum(blk.splits[:7])}
+    if where == "dt_bias":
+        blk.dt_bias[1] = value
+    else:
+        blk.w_in[3, at[where] + 1] = value
+    cache, u = _cache(blk, n, 2), n(2, 9, 64)
+    fresh = lambda: {k: v.clone() for k, v in cache.items()}
+    run = lambda: [blk.forward_single_ssd(u, fresh()), blk.step_double_ssd(u[:, 0].contiguous(), fresh())]
+    got = run()
+    monkeypatch.setattr(bm.mamba3._native, "m3_forward", lambda *a: None)
+    monkeypatch.setattr(bm.mamba3._native, "m3_step", lambda *a: None)
+    for (go, gc), (wo, wc) in zip(got, run()):
+        for a, b in [(go, wo)] + [(gc[k], wc[k]) for k in wc]:
+            assert torch.equal(a.isnan(), b.isnan()) and torch.equal(a.isinf(), b.isinf())
+            ok = b.isfinite()
+            assert not ok.any() or _close(a[ok], b[ok])
