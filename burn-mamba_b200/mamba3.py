@@ -160,8 +160,10 @@ class Mamba3:
         """-> (out [b,s,d_model], cache).  One SSD pass with the trapezoid folded into gamma / scale; B / C go
         from the projection's raw columns to the rotated per-head tensors in one kernel.  Runs natively where the kernels
         around the slot cover the block (csrc/mamba3_block.cu), else as torch ops."""
-        c = cache or {}
-        got = _native.m3_forward(self._native_args(), u_bsm, c.get("ssm"), c.get("k"), c.get("v"), c.get("angle"), chunk_len)
+        given = [cache[k] for k in ("ssm", "k", "v", "angle")] if cache else [None] * 4   # all None: the zero cache
+        got = None
+        if not cache or given[0] is not None:
+            got = _native.m3_forward(self._native_args(), u_bsm, *given, chunk_len)
         if got is not None:
             return got[0], dict(ssm=got[1], k=got[2], v=got[3], angle=got[4])
         bsz = u_bsm.shape[0]

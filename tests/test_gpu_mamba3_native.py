@@ -82,3 +82,16 @@ def test_infinities_and_nan_reach_the_output_as_in_the_unfused_block(bm, monkeyp
             assert torch.equal(a.isnan(), b.isnan()) and torch.equal(a.isinf(), b.isinf())
             ok = b.isfinite()
             assert not ok.any() or _close(a[ok], b[ok])
+
+
+@pytest.mark.parametrize("given", [("k", "v", "angle"), ("ssm", "v", "angle"), ("ssm", "k", "v")])
+def test_a_cache_without_one_of_its_tensors_is_refused(bm, given):
+    blk, n = _block(bm, 2, 64, 32, 16, 32, seed=2)
+    cache = {k: t for k, t in _cache(blk, n, 2).items() if k in given}
+    with pytest.raises(KeyError):
+        blk.forward_single_ssd(n(2, 5, 64), cache)
+    with pytest.raises(KeyError):
+        blk.step_double_ssd(n(2, 64), cache)
+    for dropped in set(("ssm", "k", "v", "angle")) - set(given):   # there, but None
+        with pytest.raises((AttributeError, TypeError)):
+            blk.forward_single_ssd(n(2, 5, 64), {**cache, dropped: None})
