@@ -1,6 +1,5 @@
 // C-ABI entry points of the chunked SSD forward (Mamba-2, Mamba-3 single / double): argument
 // validation and dispatch between the exact path and the tensor-core path.
-#include <algorithm>
 #include "common.cuh"
 #include "ssd2_tc.cuh"
 #include "ssd_exact.cuh"
@@ -184,9 +183,8 @@ extern "C" int32_t bm_workspace_status(const void* workspace, void* stream) {
 // ---------------------------------------------------------------------------------------------
 extern "C" size_t bm_ssd2_bwd_workspace_bytes(const bm_ssd2_bwd_args* a) {
     if (a == nullptr || a->batch <= 0 || a->seqlen <= 0 || a->nheads <= 0 || a->chunk_len <= 0) return 0;
-    size_t n = exact::bwd_workspace_bytes(a->batch, a->seqlen, a->nheads, a->headdim, a->state_rank, 1, a->chunk_len, true);
-    if (a->path != BM_PATH_EXACT && tc::ssd2_bwd_supported(a)) n = std::max(n, tc::ssd2_bwd_workspace_bytes(a));
-    return n;
+    if (a->path != BM_PATH_EXACT && tc::ssd2_bwd_supported(a)) return tc::ssd2_bwd_workspace_bytes(a);
+    return exact::bwd_workspace_bytes(a->batch, a->seqlen, a->nheads, a->headdim, a->state_rank, 1, a->chunk_len, true);
 }
 
 extern "C" int32_t bm_ssd2_bwd(const bm_ssd2_bwd_args* a, void* ws, size_t ws_bytes, void* stream) {
@@ -220,9 +218,8 @@ extern "C" int32_t bm_ssd2_bwd(const bm_ssd2_bwd_args* a, void* ws, size_t ws_by
 
 extern "C" size_t bm_ssd3_bwd_workspace_bytes(const bm_ssd3_bwd_args* a) {
     if (a == nullptr || a->batch <= 0 || a->seqlen <= 0 || a->nheads <= 0 || a->chunk_len <= 0) return 0;
-    size_t n = exact::bwd_workspace_bytes(a->batch, a->seqlen, a->nheads, a->headdim, a->state_rank, a->mimo_rank, a->chunk_len, false);
-    if (a->path != BM_PATH_EXACT && tc::ssd3_bwd_supported(a)) n = std::max(n, tc::ssd3_bwd_workspace_bytes(a));
-    return n;
+    if (a->path != BM_PATH_EXACT && tc::ssd3_bwd_supported(a)) return tc::ssd3_bwd_workspace_bytes(a);
+    return exact::bwd_workspace_bytes(a->batch, a->seqlen, a->nheads, a->headdim, a->state_rank, a->mimo_rank, a->chunk_len, false);
 }
 
 static int32_t ssd3_bwd(const bm_ssd3_bwd_args* a, void* ws, size_t ws_bytes, void* stream, bool single) {
