@@ -33,6 +33,7 @@
 
 #include "decode.h"
 #include "mamba3.h"
+#include "sizes.h"
 
 using at::Tensor;
 
@@ -45,6 +46,7 @@ namespace {
     X(bm_ssd3_double_bwd) X(bm_step2) X(bm_conv_step) X(bm_conv1d_silu_fwd) X(bm_rmsnorm_gated)                    \
     X(bm_mamba3_bc_prep) X(bm_selscan1_fwd) X(bm_selscan1_fwd_workspace_bytes) X(bm_selscan1_fwd_ws) X(bm_step1)   \
     X(bm_ssd3_fwd_workspace_bytes) X(bm_ssd3_single_fwd) X(bm_ssd3_double_fwd) X(bm_angle_cumsum) X(bm_step3)     \
+    X(bmx_ssd2_fwd_least_bytes) X(bmx_ssd3_fwd_least_bytes) X(bmx_ssd2_bwd_least_bytes) X(bmx_ssd3_bwd_least_bytes) \
     X(bmx_chain_status) X(bmx_chain_take_status) X(bmx_decode_slices) X(bmx_decode_linear) X(bmx_decode_norm) X(bmx_decode_conv) X(bmx_decode_state)            \
     X(bmx_decode_gated_norm) X(bmx_decode_mixer_sums) X(bmx_decode_mixer)                             \
     X(bmx_m3_coefficients) X(bmx_m3_seed) X(bmx_m3_tail) X(bmx_m3_step_covers) X(bmx_m3_step)
@@ -186,23 +188,31 @@ Workspace* find_workspace(int device, bool create) {
     const auto it = g_ws.find(key);
     return it == g_ws.end() ? nullptr : &it->second;
 }
-// f(workspace, bytes): one call of the library with a workspace of at least `nbytes`; with `status_where`, its device status
-// as well (synchronises).
+// f(workspace, bytes): one call of the library with a workspace of at least `nbytes`, or of at least `least` where the device
+// has no memory for that; with `status_where`, its device status as well (synchronises).
 template <typename F>
-void with_workspace(size_t nbytes, const Tensor& like, const char* where, const char* status_where, F f) {   // without the GIL
+void with_workspace(size_t nbytes, size_t least, const Tensor& like, const char* where, const char* status_where, F f) {   // without the GIL
     Workspace& w = *find_workspace(like.get_device(), true);
     std::lock_guard<std::mutex> lock(w.m);
     if (!w.t.defined() || (size_t)w.t.numel() < nbytes) {
-        w.t = empty({(int64_t)std::max<size_t>(nbytes, 256)}, at::kByte, like);
+        try {
+            w.t = empty({(int64_t)std::max<size_t>(nbytes, 256)}, at::kByte, like);
+        } catch (const c10::OutOfMemoryError&) {
+            if (least >= nbytes) throw;
+            if (!w.t.defined() || (size_t)w.t.numel() < least) {
+                w.t = Tensor();
+                w.t = empty({(int64_t)std::max<size_t>(least, 256)}, at::kByte, like);
+            }
+        }
         w.t.narrow(0, 0, 256).zero_();   // the status word, which not every call writes
     }
     check(f(w.t.data_ptr(), (size_t)w.t.numel()), where);
     if (status_where != nullptr) check(L.bm_workspace_status(w.t.data_ptr(), stream()), status_where);
 }
 template <typename F>
-void launch_ws(size_t nbytes, const Tensor& like, const char* where, const char* status_where, F f) {
+void launch_ws(size_t nbytes, size_t least, const Tensor& like, const char* where, const char* status_where, F f) {
     NoGil scope;
-    with_workspace(nbytes, like, where, status_where, f);
+    with_workspace(nbytes, least, like, where, status_where, f);
 }
 
 int32_t* chain_status(int device) {
@@ -292,7 +302,7 @@ FN(ssd2_fwd) {
     if (noalloc) {
         launch("bm_ssd2_fwd_noalloc", [&] { return L.bm_ssd2_fwd_noalloc(&g, stream()); });
     } else {
-        launch_ws(L.bm_ssd2_fwd_workspace_bytes(&g), x, "bm_ssd2_fwd", check_status ? "bm_ssd2_fwd (device status)" : nullptr,
+        launch_ws(L.bm_ssd2_fwd_workspace_bytes(&g), L.bmx_ssd2_fwd_least_bytes(&g), x, "bm_ssd2_fwd", check_status ? "bm_ssd2_fwd (device status)" : nullptr,
                   [&](void* ws, size_t n) { return L.bm_ssd2_fwd(&g, ws, n, stream()); });
     }
     if (want_states) return tuple({wrap(y), wrap(hf), wrap(states)});
@@ -325,7 +335,7 @@ FN(ssd2_bwd) {
     g.x = x.data_ptr(), g.dt = fptr(dt), g.a = fptr(a), g.b = b.data_ptr(), g.c = vptr(c), g.d = fptr(d), g.h0 = fptr(h0);
     g.dy = vptr(dy), g.dh_final = fptr(dhf), g.dx = fptr(dx), g.ddt = fptr(ddt), g.da = fptr(da), g.db = fptr(db), g.dc = fptr(dc);
     g.dd = d == nullptr ? nullptr : fptr(dd), g.dh0 = fptr(dh0);
-    launch_ws(L.bm_ssd2_bwd_workspace_bytes(&g), x, "bm_ssd2_bwd", check_status ? "bm_workspace_status" : nullptr,
+    launch_ws(L.bm_ssd2_bwd_workspace_bytes(&g), L.bmx_ssd2_bwd_least_bytes(&g), x, "bm_ssd2_bwd", check_status ? "bm_workspace_status" : nullptr,
               [&](void* ws, size_t n) { return L.bm_ssd2_bwd(&g, ws, n, stream()); });
     PyObject* out = PyDict_New();
     put(out, "dx", wrap(dx)), put(out, "ddt", wrap(ddt)), put(out, "da", wrap(da)), put(out, "db", wrap(db)), put(out, "dc", wrap(dc));
@@ -483,7 +493,8 @@ FN(selscan1_fwd) {
     if (serial) {
         launch("bm_selscan1_fwd", [&] { return L.bm_selscan1_fwd(&g, stream()); });
     } else {
-        launch_ws(L.bm_selscan1_fwd_workspace_bytes(&g), u, "bm_selscan1_fwd_ws", nullptr,
+        const size_t need = L.bm_selscan1_fwd_workspace_bytes(&g);
+        launch_ws(need, need, u, "bm_selscan1_fwd_ws", nullptr,
                   [&](void* ws, size_t n) { return L.bm_selscan1_fwd_ws(&g, ws, n, stream()); });
     }
     return tuple({wrap(y), wrap(hf)});
@@ -574,7 +585,7 @@ FN(ssd3_fwd) {
     g.v = v.data_ptr(), g.da = fptr(da), g.b = b.data_ptr(), g.c = vptr(c), g.gamma = fptr(gamma), g.scale = fptr(scale);
     g.h0 = fptr(h0), g.angles = fptr(ang), g.y = y.data_ptr(), g.h_final = fptr(hf);
     const std::string name = single ? "bm_ssd3_single_fwd" : "bm_ssd3_double_fwd", status_name = name + " (device status)";
-    launch_ws(L.bm_ssd3_fwd_workspace_bytes(&g), v, name.c_str(), check_status ? status_name.c_str() : nullptr,
+    launch_ws(L.bm_ssd3_fwd_workspace_bytes(&g), L.bmx_ssd3_fwd_least_bytes(&g), v, name.c_str(), check_status ? status_name.c_str() : nullptr,
               [&](void* ws, size_t n) { return (single ? L.bm_ssd3_single_fwd : L.bm_ssd3_double_fwd)(&g, ws, n, stream()); });
     return tuple({wrap(y), wrap(hf)});
     END
@@ -608,7 +619,7 @@ FN(ssd3_bwd) {
     g.mimo_rank = (int32_t)M;
     g.v = v.data_ptr(), g.da = fptr(da), g.b = b.data_ptr(), g.c = vptr(c), g.h0 = fptr(h0), g.dy = vptr(dy), g.dh_final = fptr(dhf);
     g.dv = fptr(dv), g.dda = fptr(dda), g.db = fptr(db), g.dc = fptr(dc), g.dh0 = fptr(dh0);
-    launch_ws(L.bm_ssd3_bwd_workspace_bytes(&g), v, "bm_ssd3_bwd", check_status ? "bm_workspace_status" : nullptr,
+    launch_ws(L.bm_ssd3_bwd_workspace_bytes(&g), L.bmx_ssd3_bwd_least_bytes(&g), v, "bm_ssd3_bwd", check_status ? "bm_workspace_status" : nullptr,
               [&](void* ws, size_t n) { return (single ? L.bm_ssd3_single_bwd : L.bm_ssd3_double_bwd)(&g, ws, n, stream()); });
     PyObject* out = PyDict_New();
     put(out, "dv", wrap(dv)), put(out, "dda", wrap(dda)), put(out, "db", wrap(db)), put(out, "dc", wrap(dc)), put(out, "dh0", wrap(dh0));
@@ -964,7 +975,8 @@ FN(m3_forward) {
     fa.batch = (int32_t)B, fa.seqlen = (int32_t)S, fa.nheads = (int32_t)H, fa.headdim = (int32_t)P, fa.state_rank = (int32_t)R, fa.mimo_rank = (int32_t)M;
     fa.chunk_len = (int32_t)chunk, fa.dtype = BM_DTYPE_F32, fa.v = fptr(v), fa.da = da, fa.b = fptr(bm), fa.c = fptr(cm), fa.gamma = gamma, fa.scale = scale;
     fa.h0 = ssm ? fptr(&h0) : nullptr, fa.y = fptr(y), fa.h_final = fptr(hf);
-    with_workspace(L.bm_ssd3_fwd_workspace_bytes(&fa), u, "bm_ssd3_single_fwd", nullptr, [&](void* ws, size_t n) { return L.bm_ssd3_single_fwd(&fa, ws, n, st); });
+    with_workspace(L.bm_ssd3_fwd_workspace_bytes(&fa), L.bmx_ssd3_fwd_least_bytes(&fa), u, "bm_ssd3_single_fwd", nullptr,
+                   [&](void* ws, size_t n) { return L.bm_ssd3_single_fwd(&fa, ws, n, st); });
     Tensor g = empty({B * S, b.DI}, f, u), kl = empty({B, M, H, R}, f, u), vl = empty({B, H, P}, f, u);
     check(L.bmx_m3_tail(&b.g, fptr(&y), fptr(&bm), fptr(g), fptr(kl), fptr(vl), st), "Mamba-3 block (gate)");
     Tensor out = at::mm(g, b.w_out).view({B, S, b.DM});

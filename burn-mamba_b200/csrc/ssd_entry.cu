@@ -1,6 +1,7 @@
 // C-ABI entry points of the chunked SSD forward (Mamba-2, Mamba-3 single / double): argument
 // validation and dispatch between the exact path and the tensor-core path.
 #include "common.cuh"
+#include "host/sizes.h"
 #include "ssd2_tc.cuh"
 #include "ssd_exact.cuh"
 
@@ -69,6 +70,14 @@ extern "C" size_t bm_ssd2_fwd_workspace_bytes(const bm_ssd2_fwd_args* a) {
     }
     if (a->path != BM_PATH_AUTO) return t;
     return t > 0 ? t : ex;
+}
+
+// Least workspace a call runs with (host/native.cpp): what the query above says, or less on the exact path, whose chunks grow
+// where memory is short.
+extern "C" size_t bmx_ssd2_fwd_least_bytes(const bm_ssd2_fwd_args* a) {
+    const size_t n = bm_ssd2_fwd_workspace_bytes(a);
+    if (n == 0 || ssd2_use_tensor(a)) return n;
+    return exact::least_bytes(a->batch, a->seqlen, a->nheads, a->headdim, a->state_rank, a->chunk_len, a->chunk_states != nullptr);
 }
 
 extern "C" int32_t bm_ssd2_fwd(const bm_ssd2_fwd_args* a, void* workspace, size_t workspace_bytes, void* stream) {
@@ -150,6 +159,12 @@ extern "C" size_t bm_ssd3_fwd_workspace_bytes(const bm_ssd3_fwd_args* a) {
                                   a->chunk_len, false);
 }
 
+extern "C" size_t bmx_ssd3_fwd_least_bytes(const bm_ssd3_fwd_args* a) {
+    const size_t n = bm_ssd3_fwd_workspace_bytes(a);
+    if (n == 0 || ssd3_use_tensor(a)) return n;
+    return exact::least_bytes(a->batch, a->seqlen, a->nheads, a->headdim, a->state_rank, a->chunk_len, false);
+}
+
 static int32_t ssd3_fwd(const bm_ssd3_fwd_args* a, bool single, void* ws, size_t ws_bytes, void* stream) {
     clear_error();
     if (int32_t e = validate_ssd3(a, single)) return e;
@@ -187,6 +202,12 @@ extern "C" size_t bm_ssd2_bwd_workspace_bytes(const bm_ssd2_bwd_args* a) {
     return exact::bwd_workspace_bytes(a->batch, a->seqlen, a->nheads, a->headdim, a->state_rank, 1, a->chunk_len, true);
 }
 
+extern "C" size_t bmx_ssd2_bwd_least_bytes(const bm_ssd2_bwd_args* a) {
+    const size_t n = bm_ssd2_bwd_workspace_bytes(a);
+    if (n == 0 || (a->path != BM_PATH_EXACT && tc::ssd2_bwd_supported(a))) return n;
+    return exact::bwd_least_bytes(a->batch, a->seqlen, a->nheads, a->headdim, a->state_rank, 1, a->chunk_len, true);
+}
+
 extern "C" int32_t bm_ssd2_bwd(const bm_ssd2_bwd_args* a, void* ws, size_t ws_bytes, void* stream) {
     clear_error();
     if (a == nullptr) return fail(BM_ERR_NULL_POINTER, "args is NULL");
@@ -220,6 +241,12 @@ extern "C" size_t bm_ssd3_bwd_workspace_bytes(const bm_ssd3_bwd_args* a) {
     if (a == nullptr || a->batch <= 0 || a->seqlen <= 0 || a->nheads <= 0 || a->chunk_len <= 0) return 0;
     if (a->path != BM_PATH_EXACT && tc::ssd3_bwd_supported(a)) return tc::ssd3_bwd_workspace_bytes(a);
     return exact::bwd_workspace_bytes(a->batch, a->seqlen, a->nheads, a->headdim, a->state_rank, a->mimo_rank, a->chunk_len, false);
+}
+
+extern "C" size_t bmx_ssd3_bwd_least_bytes(const bm_ssd3_bwd_args* a) {
+    const size_t n = bm_ssd3_bwd_workspace_bytes(a);
+    if (n == 0 || (a->path != BM_PATH_EXACT && tc::ssd3_bwd_supported(a))) return n;
+    return exact::bwd_least_bytes(a->batch, a->seqlen, a->nheads, a->headdim, a->state_rank, a->mimo_rank, a->chunk_len, false);
 }
 
 static int32_t ssd3_bwd(const bm_ssd3_bwd_args* a, void* ws, size_t ws_bytes, void* stream, bool single) {

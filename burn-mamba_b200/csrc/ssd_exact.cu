@@ -28,6 +28,12 @@ int inner_chunk(int Q, int M, bool want_states) {
     return q;
 }
 
+int longer_chunk(int q, int Q, bool want_states) {
+    q = q * 2 < Q ? q * 2 : Q;
+    while (want_states && Q % q) ++q;
+    return q;
+}
+
 namespace {
 
 // K1 + K3: cum_l = inclusive cumsum of da over the chunk (positions past seqlen behave as dt = 0 padding,
@@ -423,12 +429,24 @@ static size_t need_bytes(const Params& p, int q) {
     return 2 * scan_bytes(p.B, p.S, p.H, q) + (in_place ? 0 : state_bytes(p.B, p.S, p.H, p.P, p.R, q));
 }
 
-size_t workspace_bytes(int B, int S, int H, int P, int R, int M, int Q, bool want_states) {
+static size_t bytes_at(int B, int S, int H, int P, int R, int Q, bool want_states, int q) {
     Params p{};
     p.B = B, p.S = S, p.H = H, p.P = P, p.R = R, p.Qout = Q;
     float dummy;
     p.states_out = want_states ? &dummy : nullptr;
-    return need_bytes(p, inner_chunk(Q, M, want_states));
+    return need_bytes(p, q);
+}
+size_t workspace_bytes(int B, int S, int H, int P, int R, int M, int Q, bool want_states) {
+    return bytes_at(B, S, H, P, R, Q, want_states, inner_chunk(Q, M, want_states));
+}
+size_t least_bytes(int B, int S, int H, int P, int R, int Q, bool want_states) { return bytes_at(B, S, H, P, R, Q, want_states, Q); }
+
+// Shorter chunks are faster but keep more states: the chunk grows towards the caller's length until the scratch holds them.
+static int fitting_chunk(const Params& p, size_t bytes) {
+    const bool want_states = p.states_out != nullptr;
+    int q = inner_chunk(p.Q, p.M, want_states);
+    while (need_bytes(p, q) > bytes && q < p.Q) q = longer_chunk(q, p.Q, want_states);
+    return q;
 }
 
 static int32_t run_at(Params p, int q, void* workspace, size_t ws_bytes, cudaStream_t stream) {
@@ -470,7 +488,7 @@ static int32_t run_at(Params p, int q, void* workspace, size_t ws_bytes, cudaStr
 int32_t run(Params p, void* workspace, size_t ws_bytes, cudaStream_t stream) {
     p.Qout = p.Q;
     p.states_out = p.states;
-    return run_at(p, inner_chunk(p.Q, p.M, p.states_out != nullptr), workspace, ws_bytes, stream);
+    return run_at(p, fitting_chunk(p, ws_bytes), workspace, ws_bytes, stream);
 }
 
 }  // namespace exact
@@ -515,14 +533,7 @@ static int32_t noalloc_scratch_ptr(void** out) {
 int32_t run_noalloc(Params p, cudaStream_t stream) {
     p.Qout = p.Q;
     p.states_out = p.states;
-    // Shorter chunks are faster but take more scratch: where the built-in array does not hold their states, the chunk
-    // grows towards the caller's length (keeping the caller's boundaries when chunk states are wanted).
-    const bool want_states = p.states_out != nullptr;
-    int q = inner_chunk(p.Q, p.M, want_states);
-    while (need_bytes(p, q) > (size_t)BM_SSD2_NOALLOC_SCRATCH_BYTES && q < p.Q) {
-        q = q * 2 < p.Q ? q * 2 : p.Q;
-        while (want_states && p.Q % q) ++q;
-    }
+    const int q = fitting_chunk(p, (size_t)BM_SSD2_NOALLOC_SCRATCH_BYTES);
     const size_t need = need_bytes(p, q);
     if (need > (size_t)BM_SSD2_NOALLOC_SCRATCH_BYTES)
         return fail(BM_ERR_WORKSPACE_TOO_SMALL,

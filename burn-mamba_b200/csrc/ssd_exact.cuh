@@ -55,10 +55,14 @@ struct BwdParams {
     float* dh0;             // [b, h, p, r]
 };
 
+// Workspace the kernels do best with, and the least they run with: chunks grow towards the caller's length, and the states kept
+// per chunk become fewer, where the workspace given is between the two.
 size_t bwd_workspace_bytes(int B, int S, int H, int P, int R, int M, int Q, bool mamba2);
+size_t bwd_least_bytes(int B, int S, int H, int P, int R, int M, int Q, bool mamba2);
 int32_t run_bwd(BwdParams p, void* workspace, size_t workspace_bytes, cudaStream_t stream);
 
 size_t workspace_bytes(int B, int S, int H, int P, int R, int M, int Q, bool want_states);
+size_t least_bytes(int B, int S, int H, int P, int R, int Q, bool want_states);
 // Carves cum / cs / states out of `workspace` and runs K1 + K3 -> K4 -> K5 on `stream`; p.states, when given, receives the
 // state entering every chunk of p.Q steps.
 int32_t run(Params p, void* workspace, size_t workspace_bytes, cudaStream_t stream);

@@ -15,6 +15,8 @@
 //   dcum, dcs, dgs, dAend collect the scalar terms; d_da = suffix sum of dcum within the chunk.
 #include "ssd_exact_tiles.cuh"
 
+#include <algorithm>
+
 namespace bm {
 namespace exact {
 namespace {
@@ -703,15 +705,21 @@ static bool one_tile(const Params& p) { return p.P <= TP && p.R <= 128 && p.M <=
 static size_t scan_bytes(int B, int S, int H, int q) { return align_up((size_t)B * H * cdiv(S, q) * q * sizeof(float), 256); }
 static size_t state_bytes(int B, int S, int H, int P, int R, int q) { return align_up((size_t)B * cdiv(S, q) * H * P * R * sizeof(float), 256); }
 
+// Workspace of the one-tile kernel and of the block kernels at chunk length q.
+static size_t tile_bytes(int B, int S, int H, int P, int R, int q) { return 2 * scan_bytes(B, S, H, q) + 2 * state_bytes(B, S, H, P, R, q); }
+static size_t blocks_bytes(int B, int S, int H, int P, int R, int q, bool mamba2) {
+    const size_t ae = align_up((size_t)B * H * cdiv(S, q) * sizeof(float), 256);
+    const size_t outs = mamba2 ? align_up((size_t)B * S * H * sizeof(float), 256) : 0;  // internal d_da of Mamba-2
+    return 6 * scan_bytes(B, S, H, q) + 2 * state_bytes(B, S, H, P, R, q) + ae + outs;
+}
 size_t bwd_workspace_bytes(int B, int S, int H, int P, int R, int M, int Q, bool mamba2) {
     Params p{};
     p.P = P, p.R = R, p.M = M;
     const int q = inner_chunk(Q, M, false);
-    const size_t per = scan_bytes(B, S, H, q), st = state_bytes(B, S, H, P, R, q);
-    if (one_tile(p)) return 2 * per + 2 * st;
-    const size_t ae = align_up((size_t)B * H * cdiv(S, q) * sizeof(float), 256);
-    const size_t outs = mamba2 ? align_up((size_t)B * S * H * sizeof(float), 256) : 0;  // internal d_da of Mamba-2
-    return 6 * per + 2 * st + ae + outs;
+    return one_tile(p) ? tile_bytes(B, S, H, P, R, q) : blocks_bytes(B, S, H, P, R, q, mamba2);
+}
+size_t bwd_least_bytes(int B, int S, int H, int P, int R, int M, int Q, bool mamba2) {
+    return std::min(bwd_workspace_bytes(B, S, H, P, R, M, Q, mamba2), blocks_bytes(B, S, H, P, R, Q, mamba2));
 }
 
 template <typename T, bool VEC, int W>
@@ -758,14 +766,18 @@ static int32_t launch_blocks(BwdParams bp, BwdWork w, cudaStream_t stream) {
 int32_t run_bwd(BwdParams bp, void* workspace, size_t ws_bytes, cudaStream_t stream) {
     Params& p = bp.fwd;
     const bool mamba2 = bp.d_dt != nullptr;
-    const size_t need = bwd_workspace_bytes(p.B, p.S, p.H, p.P, p.R, p.M, p.Q, mamba2);
+    const size_t need = bwd_least_bytes(p.B, p.S, p.H, p.P, p.R, p.M, p.Q, mamba2);
     if (workspace == nullptr || ws_bytes < need)
         return fail(BM_ERR_WORKSPACE_TOO_SMALL, "workspace of %zu bytes given, %zu needed", ws_bytes, need);
     if (!aligned16(workspace)) return fail(BM_ERR_BAD_ALIGNMENT, "workspace is not 16-byte aligned");
     if (p.P > 128 || p.R > 256) return fail(BM_ERR_UNSUPPORTED, "backward supports headdim <= 128 and state_rank <= 256");
     if (bwd_smem_bytes(p.P, p.R) > 200 * 1024) return fail(BM_ERR_UNSUPPORTED, "headdim x state_rank too large for the backward tiles");
     if (p.B > 65535 || p.H > 65535) return fail(BM_ERR_UNSUPPORTED, "batch / nheads above 65535");
-    p.Q = inner_chunk(p.Q, p.M, false);
+    // A workspace that does not hold the states of one-tile chunks is served by the block kernels at longer chunks.
+    int q = inner_chunk(p.Q, p.M, false);
+    const bool tile = one_tile(p) && ws_bytes >= tile_bytes(p.B, p.S, p.H, p.P, p.R, q);
+    while (!tile && q < p.Q && ws_bytes < blocks_bytes(p.B, p.S, p.H, p.P, p.R, q, mamba2)) q = longer_chunk(q, p.Q, false);
+    p.Q = q;
     p.NC = (int)cdiv(p.S, p.Q);
     p.states_out = nullptr, p.h_final = nullptr;   // the final state is not an output of the backward
     const size_t per = scan_bytes(p.B, p.S, p.H, p.Q), st = state_bytes(p.B, p.S, p.H, p.P, p.R, p.Q);
@@ -775,7 +787,6 @@ int32_t run_bwd(BwdParams bp, void* workspace, size_t ws_bytes, cudaStream_t str
     p.states = reinterpret_cast<float*>(wp); wp += st;
     BwdWork w{};
     w.dstates = reinterpret_cast<float*>(wp); wp += st;
-    const bool tile = one_tile(p);
     if (!tile) {
         w.gs = reinterpret_cast<float*>(wp); wp += per;
         p.gs = w.gs;

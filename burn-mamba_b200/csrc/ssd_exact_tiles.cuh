@@ -222,6 +222,8 @@ __device__ __forceinline__ void mul_kk_upto(int nj, const float* A, int lda, con
 // ---- launches shared by the forward and the backward -----------------------------------------------------------
 // Chunk length the kernels use inside for a caller's chunk length Q: the result does not depend on it.
 int inner_chunk(int Q, int M, bool want_states);
+// The next longer one, where the scratch does not hold the states of chunks of q.
+int longer_chunk(int q, int Q, bool want_states);
 // K1 + K3: decay scan of every chunk and its state S_n (and, with `dy`, the readout gradient G_n into `dstates`); zeroes
 // `zero_n` floats at each of zero_a / zero_b on the way (accumulators of a later kernel; may be NULL).
 int32_t launch_chunk_state(const Params& p, const void* dy, float* dstates, float* zero_a, float* zero_b, int64_t zero_n, float* zero_h1,
