@@ -3,8 +3,12 @@ chunks of the caller's length need every call is served.  Tolerances as for the 
 for gradients."""
 import ctypes as C
 
+import numpy as np
 import pytest
 import torch
+
+from oracle import inputs, mamba2
+from oracle.numerics import rel_l2
 
 pytestmark = pytest.mark.gpu
 
@@ -126,3 +130,14 @@ def test_a_call_runs_where_memory_does_not_hold_what_it_asks_for(bm):
         torch.cuda.set_per_process_memory_fraction(1.0)
     torch.cuda.synchronize()
     assert all(_close(x, w, 1e-5) for x, w in zip(got, want))
+
+
+@pytest.mark.parametrize("q", [65, 130, 257])
+def test_chunk_states_at_a_chunk_length_without_large_divisors(bm, q):
+    """The caller's chunks, several tiles each, against the float64 oracle."""
+    cfg = inputs.ssd2_prefill(seed=q, batch=2, seqlen=300, nheads=2, headdim=64, state_rank=64, ngroups=1, h0_std=0.1)
+    w = {k: v.astype(np.float64) for k, v in cfg.items()}
+    want = mamba2.ssd_serial(w["x"], w["dt"], w["a"], w["b"], w["c"], w["d"], w["h0"], q, return_chunk_states=True)
+    t = {k: torch.from_numpy(np.ascontiguousarray(v, dtype=np.float32)).cuda() for k, v in cfg.items()}
+    got = bm.ops.ssd2_fwd(t["x"], t["dt"], t["a"], t["b"], t["c"], t["d"], t["h0"], chunk_len=q, path="exact", return_chunk_states=True)
+    assert all(rel_l2(g.cpu().numpy(), v) <= 1e-5 for g, v in zip(got, want))

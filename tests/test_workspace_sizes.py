@@ -46,3 +46,14 @@ def test_exact_backward_still_asks_for_the_exact_need(bm):
     n, d = _bwd2(bm, path="exact")
     assert n >= 2 * _state(d["batch"], d["seqlen"], d["nheads"], 64)
     assert _bwd2(bm, headdim=32)[0] == _bwd2(bm, path="exact", headdim=32)[0]   # a shape the tensor kernel does not cover
+
+
+@pytest.mark.parametrize("q", [65, 67, 127, 130, 254, 257])
+def test_chunk_states_at_a_chunk_length_without_large_divisors(bm, q):
+    """No divisor fills half a tile: the states live in the caller's buffer, and the workspace is two scalars per step."""
+    f = bm._ffi
+    a = f.Ssd2FwdArgs(batch=1, seqlen=4096, nheads=8, headdim=P, state_rank=R, ngroups=1, chunk_len=q, dtype=f.BM_DTYPE_F32, path=f.BM_PATH_EXACT,
+                      chunk_states=0x1000)
+    assert bm.lib.bm_ssd2_fwd_workspace_bytes(C.byref(a)) <= 2 * (8 * (4096 + q) * 4 + 256)
+    a.chunk_len = 192   # 3 x 64: chunks of one full tile, their states beside the caller's
+    assert bm.lib.bm_ssd2_fwd_workspace_bytes(C.byref(a)) >= _state(1, 4096, 8, 64)
