@@ -453,6 +453,7 @@ FN(rmsnorm_gated) {
     memset(&g, 0, sizeof g);
     g.norm_before_gate = A.flag(), g.eps = (float)A.real();
     const int64_t d = x.size(-1);
+    if (d < 1) value_error("x must have at least one column");
     const auto act = x.scalar_type();
     require_cuda(x, "x");
     g.dtype = dt_code(act);

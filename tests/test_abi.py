@@ -62,6 +62,12 @@ def test_workspace_bytes_is_pure_host(bm):
     assert bm.lib.bm_ssd2_fwd_workspace_bytes(C.byref(a)) < n
 
 
+def test_a_norm_over_no_columns_is_refused(bm):
+    import torch
+    with pytest.raises(ValueError, match="at least one column"):
+        bm.ops.rmsnorm_gated(torch.zeros(3, 0), None, torch.zeros(0))
+
+
 def test_ops_refuse_cpu_tensors(bm):
     import torch
     x = torch.zeros(1, 4, 2, 8)
