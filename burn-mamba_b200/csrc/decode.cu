@@ -557,7 +557,7 @@ extern "C" int32_t bmx_decode_mixer(const bmx_mixer* a, void* stream) {
     return launch_chained("decode_mixer", true, a->batch * a->nheads * nsplit, 256, 0, static_cast<cudaStream_t>(stream), decode_mixer_kernel, *a, nsplit);
 }
 
-extern "C" int32_t bmx_decode_conv(const bm_conv_step_args* a, const bmx_rows* in, int32_t col, int32_t first, void* stream) {
+extern "C" int32_t bmx_decode_conv(const bm_conv_step_args* a, const bmx_rows* in, int32_t col, void* stream) {
     if (int32_t e = check_rows(in)) return e;
     BM_REQUIRE_PTR(a->window);
     BM_REQUIRE_PTR(a->weight);
@@ -565,7 +565,7 @@ extern "C" int32_t bmx_decode_conv(const bm_conv_step_args* a, const bmx_rows* i
     BM_REQUIRE_PTR(a->out);
     BM_REQUIRE_PTR(a->out_b);
     BM_REQUIRE_PTR(a->out_c);
-    return launch_chained("decode_conv", !first, dim3((unsigned)cdiv(a->channels, 128), (unsigned)cdiv(a->batch, 2)), 128, 0,
+    return launch_chained("decode_conv", true, dim3((unsigned)cdiv(a->channels, 128), (unsigned)cdiv(a->batch, 2)), 128, 0,
                           static_cast<cudaStream_t>(stream), decode_conv_kernel, *a, *in, col);
 }
 

@@ -67,7 +67,7 @@ int32_t bmx_decode_norm(const void* residual, const float* residual32, const bmx
 int32_t bmx_decode_mixer_sums(int32_t batch, int32_t nheads, int32_t headdim);   /* nss of a mixer step; 0 = take the kernels apart */
 int32_t bmx_decode_mixer(const bmx_mixer* a, void* stream);
 /* bm_conv_step with its input read at column `col` of `in` */
-int32_t bmx_decode_conv(const bm_conv_step_args* a, const bmx_rows* in, int32_t col, int32_t first, void* stream);
+int32_t bmx_decode_conv(const bm_conv_step_args* a, const bmx_rows* in, int32_t col, void* stream);
 /* bm_step2 (state_rank 128) with dt read at column `col` of `in`; needs dt_bias */
 int32_t bmx_decode_state(const bm_step2_args* a, const bmx_rows* in, int32_t col, void* stream);
 /* bm_rmsnorm_gated of the dense rows a->x with z read at column 0 of `z` */

@@ -15,8 +15,7 @@ extern "C" {
 typedef struct {
     int32_t batch, seqlen, nheads, headdim, state_rank, ngroups, mimo_rank, rope_dim;
     float range, dt_min, dt_max, a_floor, eps;
-    int32_t nslice;        /* proj = sum over nslice slices, `slice` elements apart */
-    int64_t slice, ld;     /* elements between projection rows */
+    int64_t ld;            /* elements between projection rows */
     const float* proj;
     const float* dt_bias;  /* [h] */
     const float* d;        /* [h] */

@@ -837,7 +837,7 @@ FN(m2_decode) {
             memset(&ca, 0, sizeof ca);
             ca.batch = (int32_t)B, ca.channels = (int32_t)l.V, ca.kernel = 4, ca.dtype = BM_DTYPE_BF16, ca.window = fptr(l.window), ca.weight = fptr(l.conv_w);
             ca.bias = fptr(l.conv_b), ca.out = base + o_x, ca.out_b = base + o_b, ca.out_c = base + o_c, ca.split_x = (int32_t)l.DI, ca.split_bc = (int32_t)(l.G * 128);
-            check(L.bmx_decode_conv(&ca, &proj, (int32_t)l.DI, 0, st), "decode step (conv)");
+            check(L.bmx_decode_conv(&ca, &proj, (int32_t)l.DI, st), "decode step (conv)");
             bm_step2_args sa;
             memset(&sa, 0, sizeof sa);
             sa.batch = (int32_t)B, sa.nheads = (int32_t)l.H, sa.headdim = (int32_t)l.P, sa.state_rank = 128, sa.ngroups = (int32_t)l.G, sa.dtype = BM_DTYPE_BF16;
@@ -915,7 +915,7 @@ bool read_m3(PyObject* tup, const Tensor& u, M3Block& b) {
     memset(&g, 0, sizeof g);
     g.nheads = (int32_t)H, g.headdim = (int32_t)P, g.state_rank = (int32_t)R, g.ngroups = (int32_t)G, g.mimo_rank = (int32_t)M, g.rope_dim = (int32_t)rope;
     g.range = (float)fv[0], g.dt_min = (float)fv[1], g.dt_max = (float)fv[2], g.a_floor = (float)fv[3], g.eps = (float)fv[4];
-    g.nslice = 1, g.ld = b.N, g.dt_bias = fptr(&b.dt_bias), g.d = fptr(&b.d), g.b_norm = fptr(&b.b_norm), g.c_norm = fptr(&b.c_norm);
+    g.ld = b.N, g.dt_bias = fptr(&b.dt_bias), g.d = fptr(&b.d), g.b_norm = fptr(&b.b_norm), g.c_norm = fptr(&b.c_norm);
     g.b_bias = fptr(&b.b_bias), g.c_bias = fptr(&b.c_bias), g.mimo_x = b.mimo_x.defined() ? fptr(&b.mimo_x) : nullptr;
     g.mimo_z = mimo ? fptr(&b.mimo_z) : nullptr, g.mimo_o = mimo ? fptr(&b.mimo_o) : nullptr;
     return true;

@@ -16,32 +16,6 @@ namespace {
 
 __device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 
-// One value / four values of a projection row that may come in slices (all requested before the first is added).
-__device__ __forceinline__ float row1(const bmx_m3_block& a, const float* p) {
-    if (a.nslice == 1) return *p;
-    float v = 0.f;
-    for (int s0 = 0; s0 < a.nslice; s0 += 8) {
-        float t[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) t[i] = s0 + i < a.nslice ? p[(s0 + i) * a.slice] : 0.f;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) v += t[i];
-    }
-    return v;
-}
-__device__ __forceinline__ float4 row4(const bmx_m3_block& a, const float* p) {
-    if (a.nslice == 1) return ld4(p);
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int s0 = 0; s0 < a.nslice; s0 += 4) {
-        float4 t[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) t[i] = s0 + i < a.nslice ? ld4(p + (s0 + i) * a.slice) : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) v.x += t[i].x, v.y += t[i].y, v.z += t[i].z, v.w += t[i].w;
-    }
-    return v;
-}
-
 struct Columns {   // column offsets of the projection row
     int di, bc, x, b, c, dt, da, lam, rot, na;
     __device__ __forceinline__ explicit Columns(const bmx_m3_block& a) {
@@ -178,7 +152,7 @@ __global__ void __launch_bounds__(256, 2) m3_step_kernel(bmx_m3_block a, float* 
     // per-row scalars: lane j holds those of row p0 + j
     const int prow = p0 + (lane & (NR - 1));
     const bool plive = prow < P;
-    const float xl = plive ? row1(a, row + col.x + h * P + prow) : 0.f;
+    const float xl = plive ? row[col.x + h * P + prow] : 0.f;
     const float xpl = plive ? v_state[(int64_t)bh * P + prow] : 0.f;
     float mxl[M];
 #pragma unroll
@@ -189,17 +163,17 @@ __global__ void __launch_bounds__(256, 2) m3_step_kernel(bmx_m3_block a, float* 
     float tz = 0.f, tmx = 1.f, tmz = 1.f, tmo = 1.f;
     if (tp < P) {
         const int64_t w = ((int64_t)h * M + tm) * P + tp;
-        tz = row1(a, row + h * P + tp);
+        tz = row[h * P + tp];
         if (a.mimo_x) tmx = a.mimo_x[w];
         if (M > 1) tmz = a.mimo_z[w], tmo = a.mimo_o[w];
     }
-    const Trapezoid t(a, row1(a, row + col.dt + h), row1(a, row + col.da + h), row1(a, row + col.lam + h), a.dt_bias[h]);
+    const Trapezoid t(a, row[col.dt + h], row[col.da + h], row[col.lam + h], a.dt_bias[h]);
     const float alpha = expf(t.da), beta = (1.f - t.lam) * t.dt * alpha, gamma = t.lam * t.dt;
     // raw B / C rows of the head's group, one warp per row: RMS norm over r, + bias (src/mamba3/helpers.rs:82-95)
     for (int rw = warp; rw < 2 * M; rw += 8) {
         const int isc = rw / M, m = rw % M;
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (act) v = row4(a, row + (isc ? col.c : col.b) + (m * a.ngroups + g) * R + r4);
+        if (act) v = ld4(row + (isc ? col.c : col.b) + (m * a.ngroups + g) * R + r4);
         float ss = v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
@@ -216,7 +190,7 @@ __global__ void __launch_bounds__(256, 2) m3_step_kernel(bmx_m3_block a, float* 
     float th = 0.f;
     const bool ang = tid < nal;   // nal <= 64
     if (ang) {
-        th = wrap_angle(angle[(int64_t)bh * nal + tid] + t.dt * (tanhf(row1(a, row + col.rot + tid)) * (a.range * 3.14159265358979323846f)));
+        th = wrap_angle(angle[(int64_t)bh * nal + tid] + t.dt * (tanhf(row[col.rot + tid]) * (a.range * 3.14159265358979323846f)));
         sincosf(th, &sinv[tid], &cosv[tid]);
     }
     __syncthreads();
