@@ -101,6 +101,12 @@ typedef struct {
                                  (what K4 emits, src/mamba2/ssd/serial.rs:275-343); NULL = not wanted */
 } bm_ssd2_fwd_args;
 
+/* What the kernels that serve the call do best with; for this and the other SSD entry points, forward and backward.  The
+ * tensor-core path needs all of it.  The exact path keeps the states of chunks of its own (64 rows, whatever chunk_len): given
+ * less, it lengthens them towards chunk_len, and refuses (BM_ERR_WORKSPACE_TOO_SMALL) what chunks of chunk_len do not fit into
+ * either: forward two floats per step and head (steps rounded up to whole chunks) plus one state [p, r] per chunk and head, without the
+ * states when chunk_states takes them; backward six floats and two states, one float per chunk and head, and for Mamba-2 one per step
+ * and head.  Each array is rounded up to 256 bytes. */
 size_t bm_ssd2_fwd_workspace_bytes(const bm_ssd2_fwd_args* args);
 int32_t bm_ssd2_fwd(const bm_ssd2_fwd_args* args, void* workspace, size_t workspace_bytes, void* stream);
 
@@ -124,8 +130,9 @@ int32_t bm_workspace_status(const void* workspace, void* stream);
  * that loads the library holds it until the process exits); the call allocates and frees nothing.
  *   - Same arguments, layouts and results as bm_ssd2_fwd with path BM_PATH_AUTO / BM_PATH_EXACT (float32
  *     arithmetic on CUDA cores; BM_PATH_TENSOR is refused with BM_ERR_UNSUPPORTED).
- *   - Problems whose scratch need (what bm_ssd2_fwd_workspace_bytes reports for BM_PATH_EXACT) exceeds the
- *     array are refused with BM_ERR_WORKSPACE_TOO_SMALL; nothing is launched.
+ *   - Problems are refused with BM_ERR_WORKSPACE_TOO_SMALL, and nothing is launched, when the array is less than the exact
+ *     path's least workspace (stated above): the need at chunks of chunk_len, not the larger size that
+ *     bm_ssd2_fwd_workspace_bytes reports for the path's own, shorter chunks.
  *   - The first call on each device looks the array's device address up (with that device current);
  *     make that first call outside any stream capture.  The address is cached for the life of the
  *     device's primary context: after cudaDeviceReset(), or any other teardown of that context, the
