@@ -1,4 +1,5 @@
 // Version, build string and the per-thread error message of libbm_b200.
+#include <atomic>
 #include <cstdarg>
 #include <cstdio>
 
@@ -21,6 +22,17 @@ void clear_error() { g_err[0] = 0; }
 int32_t check_cuda(cudaError_t e, const char* what) {
     if (e == cudaSuccess) return BM_OK;
     return fail(BM_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
+}
+
+int sm_count() {
+    static std::atomic<int> known{0};
+    int n = known.load(std::memory_order_relaxed);
+    if (n == 0) {
+        int dev = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
+        known.store(n, std::memory_order_relaxed);
+    }
+    return n;
 }
 
 int32_t check_launch(const char* kernel) { return check_cuda(cudaGetLastError(), kernel); }

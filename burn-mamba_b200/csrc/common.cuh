@@ -19,6 +19,9 @@ int32_t check_cuda(cudaError_t e, const char* what);
 // Launch check: cudaGetLastError after a kernel launch.
 int32_t check_launch(const char* kernel);
 
+// SMs of the current device at the first call (148 where there is none).
+int sm_count();
+
 // Launch with (or without) the programmatic-dependent-launch attribute.
 template <typename... KArgs, typename... Args>
 inline int32_t launch_chained(const char* what, bool chained, dim3 grid, dim3 block, size_t smem, cudaStream_t st, void (*kernel)(KArgs...), Args&&... args) {

@@ -285,10 +285,13 @@ __global__ void __launch_bounds__(1024) decode_norm_kernel(const __nv_bfloat16* 
 // the gated norm up to its row scale, which is a factor of every output column and is applied to the out-projection's sums
 // (decode_norm_kernel).  CTA = 16 rows of one (batch, head).  The x channels' windows slide here; those of B / C have a
 // reader in every head and slide later.  State, windows and taps are fetched before the wait.
-// Taken while the (batch, head) pairs are fewer than two per SM, where a step is a chain of latencies and this replaces three
-// of them (8 layers at d_model 2560, b1: 246 -> 232 us); with more, every head redoing the conv of B / C costs more than the
-// two launches.
-constexpr int kMixRows = 16, kMixPairs = 2 * 148;
+// Taken while the (batch, head) pairs are fewer than two per SM.  It leaves the conv outputs and y in float32, where the kernels
+// apart round them to bf16 (error of a step against float64 1.7e-3 against 3.0e-3, of which the bf16 output is 1.6e-3), and it is
+// three launches in one.  That is faster only with very few pairs, since every head redoes the conv of B / C: per layer, this
+// / apart: 80 pairs 29.6 / 31.5 us (d_model 2560, b1); 128 22.9 / 21.7, 144 26.6 / 25.3, 192 24.7 / 22.4, 240 38.2 / 35.8, 288
+// 31.2 / 28.5; 320 39.3 / 36.3, 640 53.6 / 39.9.  So from about 100 pairs on the precision is paid for with 5 to 16 % of a layer's
+// time up to the line, and would be with up to a third above it.
+constexpr int kMixRows = 16;
 __global__ void __launch_bounds__(256) decode_mixer_kernel(bmx_mixer a, int nsplit) {
     constexpr int R = 128, NR = kMixRows / 8, G = 32 / NR;
     __shared__ float bc[2 * R], red[8];
@@ -474,17 +477,21 @@ extern "C" int32_t bmx_chain_take_status(int32_t* word) {
     return fail(BM_ERR_TIMEOUT, "a bounded wait of a decode step on this device ran out: that step's output and the caches it updated are not valid");
 }
 
-// A CTA takes 128 columns x one slice of K.  Where the columns alone give more than half a wave, two CTAs share an SM and
-// the slices fill those slots; else one CTA per SM with twice the stages (fewer slices for the reader to sum, the same
-// bytes in flight).  At least two 64-wide k blocks per CTA.  Batches above 8 are left to the library product: it is as fast
-// from there on (whole step, 8 layers at d_model 2560, library / streaming: b5 316 / 286 us, b9 325 / 316; 4 layers: b16
-// 185 / 191, b32 238 / 255), since the partial sums grow with the batch.
+// A CTA takes 128 columns x one slice of K, at least two 64-wide k blocks.  Few column tiles: one CTA per SM with twice the
+// stages, so that the reader sums half the slices with the same bytes in flight.  More than a third of the SMs: that would be
+// two slices or one, which leave SMs without a CTA, so two CTAs share an SM and the slices fill those slots.  Per layer at
+// batch 1, one CTA / two CTAs per SM (in-projection's tiles): 27 tiles 18.4 / 19.2 us, 35 18.6 / 20.0, 43 20.0 / 20.7;
+// 51 22.1 / 22.1, 59 24.1 / 23.7, 67 26.1 / 24.8 (batch 8: 24.5 / 24.9, 27.7 / 30.6, 25.8 / 27.2; 28.8 / 28.5, 31.6 / 31.5,
+// 33.8 / 32.0).  For an out-projection's 6 to 20 tiles the two differ by 3 % or less.
+// Batches above 8 are left to the library product: 8 rows in two planes are what the 16-row operand holds.  Up to there the
+// library takes, library / streaming per layer: d_model 768 27.4 / 18.8 us at batch 1, 26.4 / 24.7 at 8; 1536 24.9 / 21.6, 28.7 /
+// 28.1; 2560 35.3 / 29.2, 43.5 / 39.7.
 constexpr int kLinBatch = kLinRows / 2;
-static bool linear_deep(int tiles) { return tiles <= 74; }
+static bool linear_deep(int tiles) { return tiles <= sm_count() / 3; }
 extern "C" int32_t bmx_decode_slices(int32_t batch, int32_t k, int32_t n) {
     if (batch < 1 || batch > kLinBatch || k % 8 || n % 8 || k < kLinK || n < kLinCols) return 0;
     const int tiles = (int)cdiv(n, kLinCols), kb = (int)cdiv(k, kLinK);
-    return std::max(1, std::min({(linear_deep(tiles) ? 148 : 296) / tiles, kb / 2, 16}));
+    return std::max(1, std::min({(linear_deep(tiles) ? 1 : 2) * sm_count() / tiles, kb / 2, 16}));
 }
 
 extern "C" int32_t bmx_decode_linear(const void* x, int32_t planes, const void* w, float* part, int32_t batch, int32_t k, int32_t n, int32_t nslice,
@@ -549,7 +556,7 @@ extern "C" int32_t bmx_decode_norm(const void* residual, const float* residual32
 }
 
 extern "C" int32_t bmx_decode_mixer_sums(int32_t batch, int32_t nheads, int32_t headdim) {
-    return (int64_t)batch * nheads < kMixPairs ? nheads * (int32_t)cdiv(headdim, kMixRows) : 0;
+    return (int64_t)batch * nheads < 2 * sm_count() ? nheads * (int32_t)cdiv(headdim, kMixRows) : 0;
 }
 extern "C" int32_t bmx_decode_mixer(const bmx_mixer* a, void* stream) {
     if (int32_t e = check_mixer(a)) return e;

@@ -134,8 +134,10 @@ __global__ void __launch_bounds__(256) m3_tail_kernel(bmx_m3_block a, const floa
 // The step between the projections (src/mamba3/double_ssd/double_ssd/mod.rs:635-760): coefficients, QK-norm and bias,
 // rotation by the new angle, state update and readout, D skip, gate, MIMO down-projection, cache roll.  A lane owns four
 // state columns, a warp holds NR rows (all requested first) and sums its NR M readouts with one transposing butterfly.
-// NR = 8: one CTA per (b, h).  NR = 2, when the pairs are fewer than two per SM: a cluster of P / 16 CTAs, which all read the
-// caches they share (k, angle) before the first rolls them.
+// NR = 8: one CTA per (b, h).  NR = 2, while the pairs are at most one per two SMs: a cluster of P / 16 CTAs, which all read the
+// caches they share (k, angle) before the first rolls them.  Whole step, 2 / 8 rows, rank 4 N 128: 32 pairs 21.5 / 21.7 us, 64 53.1 /
+// 53.8 (d_model 1024) and 22.5 / 23.5 (d_model 256); 80 30.8 / 27.5, 96 42.4 / 38.3, 128 44.5 / 40.4, 160 51.2 / 43.1, 256 62.5 /
+// 48.4: from there on the clusters repeat the preparation of B and C for nothing.
 // ---------------------------------------------------------------------------------------------------------------
 template <int M, int NR>
 __global__ void __launch_bounds__(256, 2) m3_step_kernel(bmx_m3_block a, float* state, float* k_state, float* v_state, float* angle, float* out, int nsplit) {
@@ -266,7 +268,7 @@ int32_t launch_step(const bmx_m3_block& a, float* state, float* k_state, float* 
     const int64_t bh = (int64_t)a.batch * a.nheads;
     const int nal = std::max(a.rope_dim / 2, 1);
     const size_t smem = sizeof(float) * (size_t)(2 * ((nal + 3) & ~3) + 5 * M * a.state_rank);
-    const bool wave = bh >= 2 * 148;
+    const bool wave = bh > sm_count() / 2;
     const int nsplit = (int)cdiv(a.headdim, wave ? 64 : 16);
     cudaLaunchConfig_t cfg{};
     cudaLaunchAttribute at{};

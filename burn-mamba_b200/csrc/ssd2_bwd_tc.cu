@@ -799,17 +799,6 @@ done:
     if (warp == 2) tmem_dealloc(tmem, 512);
 }
 
-int sm_count() {
-    static int n = 0;
-    if (n == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-        if (n <= 0) n = 148;
-    }
-    return n;
-}
-
 struct BwdLayout {
     size_t off_fwd, off_cs, off_hf, off_flags, off_slots, total;
 };

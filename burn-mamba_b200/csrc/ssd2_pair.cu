@@ -793,17 +793,6 @@ done:
     if (warp == 2) tmem_dealloc(tmem, 512);
 }
 
-int num_sms_pair() {
-    static int n = 0;
-    if (n == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-        if (n <= 0) n = 148;
-    }
-    return n;
-}
-
 // Number of sequence segments per head pair: the count (up to 8) that minimises the longest CTA's work,
 // rounds of items x tiles per item, with a small charge per segment for the state hand-off.
 int choose_segments(int npairs, int tiles, int grid) {
@@ -832,7 +821,7 @@ Plan make_plan(const bm_ssd2_fwd_args* a) {
     Plan p{};
     p.npairs = a->batch * (a->nheads / 2);
     p.tiles = (int)cdiv(a->seqlen, T);
-    p.grid = num_sms_pair();
+    p.grid = sm_count();
     p.nseg = choose_segments(p.npairs, p.tiles, p.grid);
     p.tps = (p.tiles + p.nseg - 1) / p.nseg;
     const int nitems = p.npairs * p.nseg;

@@ -1089,17 +1089,6 @@ done:
     if (warp == 2) tmem_dealloc(tmem, 512);
 }
 
-int num_sms() {
-    static int n = 0;
-    if (n == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-        if (n <= 0) n = 148;
-    }
-    return n;
-}
-
 }  // namespace
 
 const char* ssd2_why_not(const bm_ssd2_fwd_args* a) {
@@ -1116,7 +1105,7 @@ bool ssd2_supported(const bm_ssd2_fwd_args* a) { return ssd2_why_not(a) == nullp
 // Workspace head shared by both launchers: status word and the CTAs' hand-over flags in the first kWsFlagBytes
 // (reset before every launch), the trace area of development builds, then one state per CTA for hand-overs.
 constexpr size_t kWsFlagBytes = 2048, kWsTraceBytes = 7 * 64 * 4 * 8;
-static size_t ws_head_bytes() { return align_up(kWsFlagBytes + kWsTraceBytes, 256) + (size_t)num_sms() * P * R * sizeof(float); }
+static size_t ws_head_bytes() { return align_up(kWsFlagBytes + kWsTraceBytes, 256) + (size_t)sm_count() * P * R * sizeof(float); }
 static void ws_head_pointers(void* workspace, Params& prm) {
     char* w = static_cast<char*>(workspace);
     prm.status = reinterpret_cast<int*>(w);
@@ -1133,7 +1122,7 @@ static int32_t launch(Params& prm, void* workspace, cudaStream_t stream) {
     cudaError_t e = cudaFuncSetAttribute(ssd2_tc_kernel<kMode, kStates>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
     if (e != cudaSuccess) return check_cuda(e, "cudaFuncSetAttribute(ssd2_tc_kernel)");
     if (int32_t r = check_cuda(cudaMemsetAsync(workspace, 0, kWsFlagBytes, stream), "cudaMemsetAsync(status)")) return r;
-    const int grid = prm.num_units < num_sms() ? prm.num_units : num_sms();
+    const int grid = prm.num_units < sm_count() ? prm.num_units : sm_count();
     if ((int64_t)prm.num_units * prm.tiles_per_unit > INT32_MAX) return fail(BM_ERR_UNSUPPORTED, "more than 2^31 tiles");
     prm.share_q = (int)((int64_t)prm.num_units * prm.tiles_per_unit / grid);
     prm.share_r = (int)((int64_t)prm.num_units * prm.tiles_per_unit % grid);

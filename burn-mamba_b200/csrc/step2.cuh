@@ -61,7 +61,8 @@ __device__ __forceinline__ void transposed_sum(float (&v)[NR], int lane) {
 // h = exp(dt A) h + dt x (x) B, y = C . h + D x (src/mamba2/mamba2.rs:907-991).  A lane owns four state columns; a warp
 // holds NR rows, all of them requested before anything waits (they are this step's own: no kernel of a chain writes them
 // before it).  The NR row sums are reduced together by a transposing butterfly.  Bound by HBM: the state in and out.
-// NR = 8 (64 rows per CTA) when there is a wave of (batch, head) pairs, else 2, which makes four times the CTAs.
+// NR = 8 (64 rows per CTA) when there are more (batch, head) pairs than SMs, else 2, which makes four times the CTAs.  bf16 P 64,
+// 2 / 8 rows: 80 pairs 4.1 / 4.8 us, 128 5.3 / 6.2, 160 to 240 6.2 / 6.2, 288 7.0 / 6.3, 320 to 400 8.2 / 8.2, 1280 18.2 / 18.3.
 template <typename T, int NR, typename DT>
 __global__ void __launch_bounds__(256) step2_rows_kernel(bm_step2_args a, DT dtsrc, int nsplit) {
     constexpr int R = 128, G = 32 / NR;
@@ -108,7 +109,7 @@ __global__ void __launch_bounds__(256) step2_rows_kernel(bm_step2_args a, DT dts
 template <typename T, typename DT>
 inline int32_t launch_step2_rows(const bm_step2_args& a, DT dt, bool chained, cudaStream_t st) {
     const int64_t bh = (int64_t)a.batch * a.nheads;
-    const bool wave = bh >= 2 * 148;
+    const bool wave = bh > sm_count();
     const int nsplit = (int)cdiv(a.headdim, wave ? 64 : 16);
     const dim3 grid((unsigned)(bh * nsplit));
     if (wave) return launch_chained("step2", chained, grid, 256, 0, st, step2_rows_kernel<T, 8, DT>, a, dt, nsplit);
