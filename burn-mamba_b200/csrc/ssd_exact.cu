@@ -548,6 +548,9 @@ int32_t run_noalloc(Params p, cudaStream_t stream) {
     if (int32_t e = noalloc_scratch_ptr(&scratch)) return e;
     // Nothing in the scratch has to start at zero: K1 writes every cumsum / column-scale entry and K3
     // writes every chunk state before anything reads them, so the previous call's contents are dead.
+    // The launches of a call go out together: two threads on one stream would otherwise use the array in turns.
+    static std::mutex launches;
+    std::lock_guard<std::mutex> lock(launches);
     return run_at(p, q, scratch, (size_t)BM_SSD2_NOALLOC_SCRATCH_BYTES, stream);
 }
 

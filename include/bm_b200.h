@@ -139,7 +139,7 @@ int32_t bm_workspace_status(const void* workspace, void* stream);
  *     library must be reloaded before this entry point is used again on that device.
  *   - All calls on a device share the one array and it keeps the previous call's contents; nothing in
  *     it needs clearing between calls, but two calls that overlap on the GPU (different streams) race
- *     on it: serialise them. */
+ *     on it: serialise them.  Calls of several host threads on one stream need no more than that. */
 #define BM_SSD2_NOALLOC_SCRATCH_BYTES (32u << 20)
 int32_t bm_ssd2_fwd_noalloc(const bm_ssd2_fwd_args* args, void* stream);
 

@@ -49,17 +49,19 @@ def test_a_call_that_waits_for_the_gpu_lets_other_threads_run(bm, what):
     assert took > 0.2 and n > 0.2 * took / 0.002, (n, took)
 
 
-def test_two_threads_on_one_stream(bm):
-    """float32: three kernels per call that hand chunk states on through the stream's workspace."""
+@pytest.mark.parametrize("entry", ["workspace", "noalloc"])
+def test_two_threads_on_one_stream(bm, entry):
+    """float32: three kernels per call that hand chunk states on through the stream's workspace, or the built-in array."""
     gens = [torch.Generator(device="cuda").manual_seed(s) for s in (1, 2)]
     ks = [_ssd(g, s) for g, s in zip(gens, (300, 500))]
-    want = [bm.ops.ssd2_fwd(**k, path="exact") for k in ks]
+    call = (lambda **k: bm.ops.ssd2_fwd(**k, path="exact")) if entry == "workspace" else bm.ops.ssd2_fwd_noalloc
+    want = [call(**k) for k in ks]
     wrong, start = [], threading.Barrier(2)
 
     def work(i):
         start.wait()
-        for _ in range(200):
-            y, h = bm.ops.ssd2_fwd(**ks[i], path="exact")
+        for _ in range(1500):
+            y, h = call(**ks[i])
             if not (torch.equal(y, want[i][0]) and torch.equal(h, want[i][1])):
                 wrong.append(i)
 
