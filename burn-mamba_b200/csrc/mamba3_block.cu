@@ -2,7 +2,7 @@
 // gate and down-projection of a prompt, and the whole step of one token between the two projections.
 //
 // Each replaces a run of elementwise passes over [b, s, m, h, p] or [b, h] tensors: 50 launches of a prompt became 4, 52 of a
-// step became 1.  Measured: prompt b2 L389 d_model 1024 rank 4, the block 862 -> 566 us; step b64 at the same width 406 -> 122 us
+// step became 1.  Measured: prompt b2 L389 d_model 1024 rank 4, the block 862 -> 566 us; step b64 at the same width 406 -> 119 us
 // (52 us of it this step kernel: 134 MB of state in and out, bound by the latencies of its phases at two CTAs per SM).
 #include "common.cuh"
 #include "host/mamba3.h"
@@ -44,7 +44,7 @@ struct Trapezoid {   // src/mamba3/helpers.rs:42-73
     }
 };
 
-// One CTA per token.  Bound by the store of v.
+// One CTA per token.  Waits on its loads (43 % of DRAM, b4 L1024 H32 rank 4).
 __global__ void __launch_bounds__(256) m3_coefficients_kernel(bmx_m3_block a, float* dt, float* da, float* gamma, float* scale, float* v, float* rot) {
     const Columns col(a);
     const int64_t tok = blockIdx.x;
@@ -99,7 +99,8 @@ __device__ __forceinline__ float gated(float y, float x, float d, float z, float
     return fmaf(d, x * mx, y) * silu_f32(z * mz) * mo;
 }
 
-// One CTA per token: src/mamba3/single_ssd/single_ssd/mod.rs:291-337.  Bound by the load of y.
+// One CTA per token: src/mamba3/single_ssd/single_ssd/mod.rs:291-337.  The gates take 59 % of the issue
+// slots (36 % of DRAM, b4 L1024 H32 rank 4).
 __global__ void __launch_bounds__(256) m3_tail_kernel(bmx_m3_block a, const float* y, const float* b_rot, float* out, float* k_last, float* v_last) {
     const Columns col(a);
     const int64_t tok = blockIdx.x, b = tok / a.seqlen;

@@ -52,8 +52,9 @@ __device__ __forceinline__ void put4(float* row, int c, int width, float a, floa
 }
 
 // The whole backward of one chunk that is one tile (Q M <= 64 rows, P <= 64, R <= W): the eight products of the header
-// comment, each operand staged once, and the scalar gradients up to the finished suffix sum.  Bound by the float32 pipe
-// (1.6 M multiply-adds per tile at P = R = 64, 2.7 M at R = 128); one CTA per SM (122 / 171 KB of shared memory).
+// comment, each operand staged once, and the scalar gradients up to the finished suffix sum: 1.6 M multiply-adds per tile at
+// P = R = 64, 2.7 M at R = 128, fed from shared memory (that pipe 56 % busy, the float32 pipe 38 %) by the eight warps of the
+// one CTA that fits an SM (122 / 171 KB of shared memory).
 // Measured at b2 L500 H8 P64 N64: 23 us, against 730 us for the column, row and finalise kernels below; the whole
 // backward 1290 -> 45 us.
 template <typename T, bool VEC, int W>

@@ -185,9 +185,9 @@ def stack_step(blocks, norm_gammas, caches, x_bm, check_status=False):
     """One decode step through a stack of pre-norm residual layers, the default (no class latents, plain
     residual) path of Layers::step / Layer::step_one (src/modules/layers.rs:427-497,
     src/modules/layer.rs:224-229): x <- x + block.step(norm(x)).  `caches` is one Mamba2Cache per layer,
-    updated in place.  Returns the output of the last layer [b, d_model].  Per layer this is six launches
-    (norm with the residual sum, in-projection, conv step, state step, gated norm, out-projection), chained so that each
-    starts while the one before it runs; none of them depends on the host, so the whole step can be replayed from a
+    updated in place.  Returns the output of the last layer [b, d_model].  Per layer this is four launches
+    (norm with the residual sum, in-projection, mixer, out-projection) up to a batch of 8 and 296 (row, head) pairs, and six above
+    (conv step, state step and gated norm apart), chained so that each starts while the one before it runs; none of them depends on the host, so the whole step can be replayed from a
     CUDA graph.  Stacks the native chain does not cover run layer by layer.  `check_status` as in `Mamba2.step`."""
     chain = [blk._chain(cache, gamma) for blk, gamma, cache in zip(blocks, norm_gammas, caches)]
     out = _native.m2_decode(chain, x_bm, None, ops.DIV_EPS[torch.bfloat16], check_status)
